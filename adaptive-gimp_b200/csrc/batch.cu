@@ -363,8 +363,7 @@ agimp_status batch_step(agimp_batch* b, float dt, int n, cudaStream_t use, cudaE
 
 namespace {
 struct GatherSrc {
-  const float* x;
-  const int32_t* id;
+  Particles P;
   long long N, off;
 };
 
@@ -383,9 +382,11 @@ __global__ void k_gather_x(const int* ofs, int n, const GatherSrc* src, float* o
   const GatherSrc g = src[lo];
   const int bid = cta - ofs[lo], nblk = ofs[lo + 1] - ofs[lo];
   for (long long s = bid * (long long)blockDim.x + threadIdx.x; s < g.N; s += (long long)nblk * blockDim.x) {
-    const long long o = (g.off + g.id[s]) * D;
+    const long long o = (g.off + g.P.id[s]) * D;
+    float x[D];
+    load_x<D>(g.P, s, x);
 #pragma unroll
-    for (int d = 0; d < D; ++d) out[o + d] = g.x[d * g.N + s];
+    for (int d = 0; d < D; ++d) out[o + d] = x[d];
   }
 }
 }  // namespace
@@ -424,7 +425,7 @@ agimp_status batch_positions_async(agimp_batch* b, float* x, cudaStream_t use) {
   long long off = 0;
   for (int i = 0; i < n; ++i) {
     agimp_sim* s = b->sims[i];
-    hs[i] = GatherSrc{s->buf[s->par].x, s->buf[s->par].id, (long long)s->c.N, off};
+    hs[i] = GatherSrc{s->buf[s->par], (long long)s->c.N, off};
     off += s->c.N;
   }
   cudaStream_t gs = b->gather;
@@ -453,15 +454,14 @@ agimp_status batch_positions_async(agimp_batch* b, float* x, cudaStream_t use) {
 
 namespace {
 struct ScatterDst {
-  void* dst;           // the scene's field: comps x N, slot-major per component
-  const int32_t* id;   // storage slot -> caller index
+  Particles P;
   long long N, off;    // particles; first index in the concatenated arrays
 };
 
-// every scene's field from the concatenated caller arrays (particle-major,
-// comps values each, scenes in batch order) into its storage
-template <typename T>
-__global__ void k_scatter_in(const int* ofs, int n, const ScatterDst* tab, const T* src, int comps) {
+// every scene's particles from the concatenated caller arrays (scenes in batch
+// order); one pass moves every field of the call
+template <int D>
+__global__ void k_scatter_in(const int* ofs, int n, const ScatterDst* tab, Fields f) {
   const int cta = (int)blockIdx.x;
   int lo = 0, hi = n - 1;
   while (lo < hi) {
@@ -472,12 +472,9 @@ __global__ void k_scatter_in(const int* ofs, int n, const ScatterDst* tab, const
       hi = mid - 1;
   }
   const ScatterDst t = tab[lo];
-  T* dst = (T*)t.dst;
   const int bid = cta - ofs[lo], nblk = ofs[lo + 1] - ofs[lo];
-  for (long long s = bid * (long long)blockDim.x + threadIdx.x; s < t.N; s += (long long)nblk * blockDim.x) {
-    const long long o = (t.off + t.id[s]) * comps;
-    for (int c = 0; c < comps; ++c) dst[c * t.N + s] = src[o + c];
-  }
+  for (long long s = bid * (long long)blockDim.x + threadIdx.x; s < t.N; s += (long long)nblk * blockDim.x)
+    fields_in<D>(t.P, s, f, t.off + t.P.id[s]);
 }
 }  // namespace
 
@@ -501,8 +498,6 @@ agimp_status batch_set_particles(agimp_batch* b, const float* x, const float* v,
     s->bins_valid = false;
   }
   if (b->read_pending) BCK(cudaStreamWaitEvent(use, b->ev_read, 0));
-  const void* fields[7] = {x, v, F, C, m, Jp, g};
-  const int comps[7] = {D, D, D * D, D * D, 1, 1, 1};
   const size_t need = (size_t)std::max<long long>(tot, 1) * D * D;
   if (memory == AGIMP_MEM_HOST && need > b->ustage_floats) {
     if (b->ustage) BCK(cudaFree(b->ustage));
@@ -512,35 +507,48 @@ agimp_status batch_set_particles(agimp_batch* b, const float* x, const float* v,
     b->ustage_floats = need;
   }
   if (!b->utab) {
-    BCK(cudaMalloc(&b->utab, 7 * sizeof(ScatterDst) * n));
-    BCK(cudaMallocHost(&b->utab_h, 7 * sizeof(ScatterDst) * n));
+    BCK(cudaMalloc(&b->utab, sizeof(ScatterDst) * n));
+    BCK(cudaMallocHost(&b->utab_h, sizeof(ScatterDst) * n));
   }
   ScatterDst* th = (ScatterDst*)b->utab_h;
   long long off = 0;
   for (int i = 0; i < n; ++i) {
     agimp_sim* s = b->sims[i];
-    const Particles& P = s->buf[s->par];
-    void* dst[7] = {P.x, P.v, P.F, P.C, P.m, P.Jp, P.g};
-    for (int f = 0; f < 7; ++f) th[f * n + i] = ScatterDst{dst[f], P.id, (long long)s->c.N, off};
+    th[i] = ScatterDst{s->buf[s->par], (long long)s->c.N, off};
     off += s->c.N;
   }
-  BCK(cudaMemcpyAsync(b->utab, th, 7 * sizeof(ScatterDst) * n, cudaMemcpyHostToDevice, use));
+  BCK(cudaMemcpyAsync(b->utab, th, sizeof(ScatterDst) * n, cudaMemcpyHostToDevice, use));
   const int G = b->nct[MAP_G];
-  for (int f = 0; f < 7; ++f) {
-    if (!fields[f] || tot == 0) continue;
-    const void* src = fields[f];
-    if (memory == AGIMP_MEM_HOST) {
-      // one field at a time through the staging buffer (stream order keeps
-      // the next field's copy behind this field's scatter)
-      BCK(cudaMemcpyAsync(b->ustage, src, tot * comps[f] * sizeof(float), cudaMemcpyHostToDevice, use));
-      src = b->ustage;
-    }
-    const ScatterDst* td = (const ScatterDst*)b->utab + (size_t)f * n;
-    if (f == 6)
-      k_scatter_in<int32_t><<<G, 256, 0, use>>>(b->dofs + MAP_G * (n + 1), n, td, (const int32_t*)src, 1);
+  const int* ofs = b->dofs + MAP_G * (n + 1);
+  const ScatterDst* td = (const ScatterDst*)b->utab;
+  auto scatter = [&](const Fields& f) {
+    if (D == 2)
+      k_scatter_in<2><<<G, 256, 0, use>>>(ofs, n, td, f);
     else
-      k_scatter_in<float><<<G, 256, 0, use>>>(b->dofs + MAP_G * (n + 1), n, td, (const float*)src, comps[f]);
-    BCK(cudaGetLastError());
+      k_scatter_in<3><<<G, 256, 0, use>>>(ofs, n, td, f);
+    return cudaGetLastError();
+  };
+  const Fields all{(float*)x, (float*)v, (float*)F, (float*)C, (float*)m, (float*)Jp, (int32_t*)g, nullptr};
+  if (tot && memory == AGIMP_MEM_DEVICE) {
+    BCK(scatter(all));
+  } else if (tot) {
+    // host arrays: one field at a time through the staging buffer (stream
+    // order keeps the next field's copy behind this field's scatter)
+    auto field = [&](auto slot, int comps) -> cudaError_t {
+      const void* src = all.*slot;
+      if (!src) return cudaSuccess;
+      Fields f = {};
+      f.*slot = (decltype(f.*slot + 0))b->ustage;
+      const cudaError_t e = cudaMemcpyAsync(b->ustage, src, tot * comps * sizeof(float), cudaMemcpyHostToDevice, use);
+      return e != cudaSuccess ? e : scatter(f);
+    };
+    BCK(field(&Fields::x, D));
+    BCK(field(&Fields::v, D));
+    BCK(field(&Fields::F, D * D));
+    BCK(field(&Fields::C, D * D));
+    BCK(field(&Fields::m, 1));
+    BCK(field(&Fields::Jp, 1));
+    BCK(field(&Fields::g, 1));
   }
   for (agimp_sim* s : b->sims) {
     BCK(cudaEventRecord(s->ev_state, use));  // later asynchronous readbacks follow the upload
@@ -596,20 +604,13 @@ struct Saved {
 };
 
 size_t state_bytes(const agimp_sim* s) {
-  const size_t N = s->c.N, D = s->c.dim;
-  return (2 * D + 2 * D * D + 5) * N * 4;
+  return state_quads(s->c.dim, s->c.N) * sizeof(float4) + (size_t)s->c.N * 8;
 }
 
 template <class F>
 void for_each_array(agimp_sim* s, const Particles& P, F f) {
-  const size_t N = s->c.N, D = s->c.dim;
-  f(P.x, D * N * 4);
-  f(P.v, D * N * 4);
-  f(P.F, D * D * N * 4);
-  f(P.C, D * D * N * 4);
-  f(P.m, N * 4);
-  f(P.Jp, N * 4);
-  f(P.g, N * 4);
+  const size_t N = s->c.N;
+  f(P.s, state_quads(s->c.dim, N) * sizeof(float4));
   f(P.fl, N * 4);
   f(P.id, N * 4);
 }

@@ -82,37 +82,19 @@ struct StreamUse {
 };
 
 // Caller arrays are in the caller's particle order; storage slot i holds
-// particle id[i].
-__global__ void k_aos_to_soa(const float* __restrict__ aos, const int32_t* __restrict__ id, float* __restrict__ soa,
-                             long long n, int comps) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * comps;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long slot = i / comps;
-    const int c = (int)(i % comps);
-    soa[c * n + slot] = aos[(long long)id[slot] * comps + c];
-  }
-}
-
-__global__ void k_soa_to_aos(const float* __restrict__ soa, const int32_t* __restrict__ id, float* __restrict__ aos,
-                             long long n, int comps) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n * comps;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long slot = i / comps;
-    const int c = (int)(i % comps);
-    aos[(long long)id[slot] * comps + c] = soa[c * n + slot];
-  }
-}
-
-__global__ void k_i32_in(const int32_t* __restrict__ src, const int32_t* __restrict__ id, int32_t* __restrict__ dst,
-                         long long n) {
+// particle id[i].  One pass moves every field of the call.
+template <int D>
+__global__ void k_fields_in(Particles P, Fields f, long long n) {
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[i] = src[id[i]];
+    fields_in<D>(P, i, f, P.id[i]);
 }
 
-__global__ void k_i32_out(const int32_t* __restrict__ src, const int32_t* __restrict__ id, int32_t* __restrict__ dst,
-                          long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dst[id[i]] = src[i];
+template <int D, bool MAT>
+__global__ void __launch_bounds__(32 * FIELD_WARPS) k_fields_out(Particles P, Fields f, long long n) {
+  __shared__ float s[FIELD_WARPS][MAT ? 32 * FIELD_STRIDE : 1];
+  const int warp = threadIdx.x >> 5;
+  for (long long i = 32 * (blockIdx.x * (long long)FIELD_WARPS + warp); i < n; i += 32ll * gridDim.x * FIELD_WARPS)
+    fields_out<D, MAT>(P, i, n, f, s[warp]);
 }
 
 // Bin key of every particle in the last substep (adaptive_gimp.py:208-216:
@@ -148,9 +130,13 @@ __global__ void k_get_bins(Ctx c, const int32_t* __restrict__ id, unsigned long 
   }
 }
 
-__global__ void k_iota(int32_t* __restrict__ id, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    id[i] = (int32_t)i;
+// a new simulator's particles: caller index = slot, Jp = 1
+template <int D>
+__global__ void k_first_state(Particles P, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    P.id[i] = (int32_t)i;
+    ((float*)P.s)[pword<D>(i, PWord<D>::JP)] = 1.f;
+  }
 }
 
 template <int D>
@@ -201,6 +187,44 @@ int gs_blocks(long long n) {
   long long b = (n + 255) / 256;
   if (b > 65535) b = 65535;
   return (int)(b < 1 ? 1 : b);
+}
+
+// launches the move of `f`'s fields between the caller's device arrays and buffer P
+cudaError_t move_fields(agimp_sim* s, const Particles& P, const Fields& f, bool in, cudaStream_t st) {
+  const long long N = s->c.N;
+  if (N == 0) return cudaSuccess;
+  const int G = gs_blocks(N);
+  if (s->c.dim == 2) {
+    if (in)
+      k_fields_in<2><<<G, 256, 0, st>>>(P, f, N);
+    else
+      k_fields_out<2, false><<<G, 32 * FIELD_WARPS, 0, st>>>(P, f, N);
+  } else {
+    if (in)
+      k_fields_in<3><<<G, 256, 0, st>>>(P, f, N);
+    else if (f.F || f.C)
+      k_fields_out<3, true><<<G, 32 * FIELD_WARPS, 0, st>>>(P, f, N);
+    else
+      k_fields_out<3, false><<<G, 32 * FIELD_WARPS, 0, st>>>(P, f, N);
+  }
+  return cudaGetLastError();
+}
+
+// Host arrays go through the staging buffer one field at a time (stream order
+// keeps the next field's copy behind this field's kernel).
+template <typename T>
+agimp_status host_field(agimp_sim* s, T* Fields::*slot, const T* src, T* dst, int comps, cudaStream_t st) {
+  const size_t bytes = (size_t)s->c.N * comps * sizeof(T);
+  if (bytes == 0) return AGIMP_OK;
+  Fields f = {};
+  f.*slot = (T*)s->staging;
+  if (src) CK(cudaMemcpyAsync(s->staging, src, bytes, cudaMemcpyHostToDevice, st));
+  CK(move_fields(s, s->buf[s->par], f, src != nullptr, st));
+  if (dst) {
+    CK(cudaMemcpyAsync(dst, s->staging, bytes, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+  }
+  return AGIMP_OK;
 }
 
 }  // namespace
@@ -383,30 +407,14 @@ agimp_status agimp_create(const agimp_params* p, int32_t device, agimp_sim** out
   AL(c.proj, N + 1);
   for (int k = 0; k < 2; ++k) {
     Particles& P = s->buf[k];
-    AL(P.x, D * N + 1);
-    AL(P.v, D * N + 1);
-    AL(P.F, D * D * N + 1);
-    AL(P.C, D * D * N + 1);
-    AL(P.m, N + 1);
-    AL(P.Jp, N + 1);
-    AL(P.g, N + 1);
+    AL(P.s, state_quads(D, N) + 1);
     AL(P.fl, N + 1);
     AL(P.id, N + 1);
-    cudaMemset(P.x, 0, (D * N + 1) * sizeof(float));
-    cudaMemset(P.v, 0, (D * N + 1) * sizeof(float));
-    cudaMemset(P.F, 0, (D * D * N + 1) * sizeof(float));
-    cudaMemset(P.C, 0, (D * D * N + 1) * sizeof(float));
-    cudaMemset(P.m, 0, (N + 1) * sizeof(float));
-    cudaMemset(P.g, 0, (N + 1) * sizeof(int32_t));
+    cudaMemset(P.s, 0, state_quads(D, N) * sizeof(float4));
     cudaMemset(P.fl, 0xff, (N + 1) * sizeof(int32_t));
   }
   s->staging_floats = std::max<size_t>((size_t)1 << 20, (size_t)(D * D * N));
   AL(s->staging, s->staging_floats);
-  {
-    // Jp starts at 1
-    std::vector<float> ones(N + 1, 1.0f);
-    cudaMemcpy(s->buf[0].Jp, ones.data(), (N + 1) * sizeof(float), cudaMemcpyHostToDevice);
-  }
 #undef AL
   if (cudaStreamCreateWithFlags(&s->internal, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&s->ev_in, cudaEventDisableTiming) != cudaSuccess ||
@@ -422,9 +430,11 @@ agimp_status agimp_create(const agimp_params* p, int32_t device, agimp_sim** out
     agimp_destroy(s);
     return AGIMP_CUDA_ERROR;
   }
-  // storage slot i starts with caller particle i (on the simulator's own
-  // stream; the synchronisation below orders it before any use)
-  if (N) k_iota<<<gs_blocks(N), 256, 0, s->internal>>>(s->buf[0].id, N);
+  // (the memsets above ran on the legacy default stream; the synchronisation
+  // below orders this before any use)
+  cudaDeviceSynchronize();
+  if (N && D == 2) k_first_state<2><<<gs_blocks(N), 256, 0, s->internal>>>(s->buf[0], N);
+  if (N && D == 3) k_first_state<3><<<gs_blocks(N), 256, 0, s->internal>>>(s->buf[0], N);
   s->self = new agimp_batch();
   s->self->sims.push_back(s);
   s->self->single = true;
@@ -470,57 +480,6 @@ agimp_status agimp_destroy(agimp_sim* s) {
   return AGIMP_OK;
 }
 
-static agimp_status upload_soa(agimp_sim* s, const float* src, float* dst, int comps, int memory, cudaStream_t st) {
-  const long long N = s->c.N;
-  if (N == 0) return AGIMP_OK;
-  const float* aos = src;
-  if (memory == AGIMP_MEM_HOST) {
-    CK(cudaMemcpyAsync(s->staging, src, N * comps * sizeof(float), cudaMemcpyHostToDevice, st));
-    aos = s->staging;
-  }
-  k_aos_to_soa<<<gs_blocks(N * comps), 256, 0, st>>>(aos, s->buf[s->par].id, dst, N, comps);
-  CK(cudaGetLastError());
-  return AGIMP_OK;
-}
-
-static agimp_status download_soa(agimp_sim* s, const float* src, float* dst, int comps, int memory, cudaStream_t st) {
-  const long long N = s->c.N;
-  if (N == 0) return AGIMP_OK;
-  float* aos = (memory == AGIMP_MEM_HOST) ? s->staging : dst;
-  k_soa_to_aos<<<gs_blocks(N * comps), 256, 0, st>>>(src, s->buf[s->par].id, aos, N, comps);
-  CK(cudaGetLastError());
-  if (memory == AGIMP_MEM_HOST) {
-    CK(cudaMemcpyAsync(dst, s->staging, N * comps * sizeof(float), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-  }
-  return AGIMP_OK;
-}
-
-static agimp_status copy_i32(agimp_sim* s, const int32_t* src, int32_t* dst, int to_dev, int memory, cudaStream_t st) {
-  const long long N = s->c.N;
-  if (N == 0) return AGIMP_OK;
-  const int32_t* id = s->buf[s->par].id;
-  int32_t* tmp = (int32_t*)s->staging;
-  if (to_dev) {
-    const int32_t* from = src;
-    if (memory == AGIMP_MEM_HOST) {
-      CK(cudaMemcpyAsync(tmp, src, N * sizeof(int32_t), cudaMemcpyHostToDevice, st));
-      from = tmp;
-    }
-    k_i32_in<<<gs_blocks(N), 256, 0, st>>>(from, id, dst, N);
-    CK(cudaGetLastError());
-  } else {
-    int32_t* to = memory == AGIMP_MEM_HOST ? tmp : dst;
-    k_i32_out<<<gs_blocks(N), 256, 0, st>>>(src, id, to, N);
-    CK(cudaGetLastError());
-    if (memory == AGIMP_MEM_HOST) {
-      CK(cudaMemcpyAsync(dst, tmp, N * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-    }
-  }
-  return AGIMP_OK;
-}
-
 agimp_status agimp_set_particles(agimp_sim* s, const float* x, const float* v, const float* F, const float* C,
                                  const float* m, const int32_t* g, const float* Jp, int32_t memory, void* stream) {
   if (!s || (memory != AGIMP_MEM_DEVICE && memory != AGIMP_MEM_HOST)) return fail(s, AGIMP_INVALID_ARG, "bad args");
@@ -529,15 +488,26 @@ agimp_status agimp_set_particles(agimp_sim* s, const float* x, const float* v, c
   wait_readback(s, s->par, su.use);  // the upload overwrites the state being read
   s->bins_valid = false;
   const int D = s->c.dim;
-  const Particles& P = s->buf[s->par];
-  agimp_status r;
-  if (x && (r = upload_soa(s, x, P.x, D, memory, su.use))) return r;
-  if (v && (r = upload_soa(s, v, P.v, D, memory, su.use))) return r;
-  if (F && (r = upload_soa(s, F, P.F, D * D, memory, su.use))) return r;
-  if (C && (r = upload_soa(s, C, P.C, D * D, memory, su.use))) return r;
-  if (m && (r = upload_soa(s, m, P.m, 1, memory, su.use))) return r;
-  if (Jp && (r = upload_soa(s, Jp, P.Jp, 1, memory, su.use))) return r;
-  if (g && (r = copy_i32(s, g, P.g, 1, memory, su.use))) return r;
+  if (memory == AGIMP_MEM_DEVICE) {
+    Fields f = {};
+    f.x = (float*)x;
+    f.v = (float*)v;
+    f.F = (float*)F;
+    f.C = (float*)C;
+    f.m = (float*)m;
+    f.Jp = (float*)Jp;
+    f.g = (int32_t*)g;
+    CK(move_fields(s, s->buf[s->par], f, true, su.use));
+  } else {
+    agimp_status r;
+    if (x && (r = host_field<float>(s, &Fields::x, x, nullptr, D, su.use))) return r;
+    if (v && (r = host_field<float>(s, &Fields::v, v, nullptr, D, su.use))) return r;
+    if (F && (r = host_field<float>(s, &Fields::F, F, nullptr, D * D, su.use))) return r;
+    if (C && (r = host_field<float>(s, &Fields::C, C, nullptr, D * D, su.use))) return r;
+    if (m && (r = host_field<float>(s, &Fields::m, m, nullptr, 1, su.use))) return r;
+    if (Jp && (r = host_field<float>(s, &Fields::Jp, Jp, nullptr, 1, su.use))) return r;
+    if (g && (r = host_field<int32_t>(s, &Fields::g, g, nullptr, 1, su.use))) return r;
+  }
   CK(cudaEventRecord(s->ev_state, su.use));  // later asynchronous readbacks follow the upload
   s->state_marked = true;
   if (memory == AGIMP_MEM_HOST) CK(cudaStreamSynchronize(su.use));  // host buffers may be reused on return
@@ -550,16 +520,19 @@ agimp_status agimp_get_particles(agimp_sim* s, float* x, float* v, float* F, flo
   CK(cudaSetDevice(s->device));
   StreamUse su(s, stream);
   const int D = s->c.dim;
-  const Particles& P = s->buf[s->par];
+  if (memory == AGIMP_MEM_DEVICE) {
+    CK(move_fields(s, s->buf[s->par], Fields{x, v, F, C, m, Jp, g, fl}, false, su.use));
+    return AGIMP_OK;
+  }
   agimp_status r;
-  if (x && (r = download_soa(s, P.x, x, D, memory, su.use))) return r;
-  if (v && (r = download_soa(s, P.v, v, D, memory, su.use))) return r;
-  if (F && (r = download_soa(s, P.F, F, D * D, memory, su.use))) return r;
-  if (C && (r = download_soa(s, P.C, C, D * D, memory, su.use))) return r;
-  if (m && (r = download_soa(s, P.m, m, 1, memory, su.use))) return r;
-  if (Jp && (r = download_soa(s, P.Jp, Jp, 1, memory, su.use))) return r;
-  if (g && (r = copy_i32(s, P.g, g, 0, memory, su.use))) return r;
-  if (fl && (r = copy_i32(s, P.fl, fl, 0, memory, su.use))) return r;
+  if (x && (r = host_field<float>(s, &Fields::x, nullptr, x, D, su.use))) return r;
+  if (v && (r = host_field<float>(s, &Fields::v, nullptr, v, D, su.use))) return r;
+  if (F && (r = host_field<float>(s, &Fields::F, nullptr, F, D * D, su.use))) return r;
+  if (C && (r = host_field<float>(s, &Fields::C, nullptr, C, D * D, su.use))) return r;
+  if (m && (r = host_field<float>(s, &Fields::m, nullptr, m, 1, su.use))) return r;
+  if (Jp && (r = host_field<float>(s, &Fields::Jp, nullptr, Jp, 1, su.use))) return r;
+  if (g && (r = host_field<int32_t>(s, &Fields::g, nullptr, g, 1, su.use))) return r;
+  if (fl && (r = host_field<int32_t>(s, &Fields::fl, nullptr, fl, 1, su.use))) return r;
   return AGIMP_OK;
 }
 
@@ -630,7 +603,6 @@ agimp_status agimp_get_particles_async(agimp_sim* s, float* x, float* v, float* 
     CK(cudaMalloc(&s->astage, 2 * need * sizeof(float)));
     s->astage_floats = need;
   }
-  float* const st0 = s->astage + (size_t)slot * s->astage_floats;
   struct Copy {
     void* dst;
     const float* src;
@@ -638,29 +610,25 @@ agimp_status agimp_get_particles_async(agimp_sim* s, float* x, float* v, float* 
   };
   Copy copies[8];
   int ncopy = 0;
-  float* st = st0;
-  auto field = [&](const float* src, float* dst, int comps) -> cudaError_t {
-    if (!dst || !N) return cudaSuccess;
-    k_soa_to_aos<<<gs_blocks(N * comps), 256, 0, gs>>>(src, P.id, st, N, comps);
-    copies[ncopy++] = {dst, st, N * comps * sizeof(float)};
+  float* st = s->astage + (size_t)slot * s->astage_floats;
+  // the field's place in the staging slot, null when it was not asked for
+  auto field = [&](void* dst, int comps) -> float* {
+    if (!dst || !N) return nullptr;
+    float* at = st;
+    copies[ncopy++] = {dst, at, N * comps * sizeof(float)};
     st += N * comps;
-    return cudaGetLastError();
+    return at;
   };
-  auto ifield = [&](const int32_t* src, int32_t* dst) -> cudaError_t {
-    if (!dst || !N) return cudaSuccess;
-    k_i32_out<<<gs_blocks(N), 256, 0, gs>>>(src, P.id, (int32_t*)st, N);
-    copies[ncopy++] = {dst, st, N * sizeof(int32_t)};
-    st += N;
-    return cudaGetLastError();
-  };
-  CK(field(P.x, x, D));
-  CK(field(P.v, v, D));
-  CK(field(P.F, F, D * D));
-  CK(field(P.C, C, D * D));
-  CK(field(P.m, m, 1));
-  CK(field(P.Jp, Jp, 1));
-  CK(ifield(P.g, g));
-  CK(ifield(P.fl, fl));
+  Fields f = {};
+  f.x = field(x, D);
+  f.v = field(v, D);
+  f.F = field(F, D * D);
+  f.C = field(C, D * D);
+  f.m = field(m, 1);
+  f.Jp = field(Jp, 1);
+  f.g = (int32_t*)field(g, 1);
+  f.fl = (int32_t*)field(fl, 1);
+  CK(move_fields(s, P, f, false, gs));
   // the state has been read: a substep may overwrite it from here on
   CK(cudaEventRecord(s->ev_read[k], gs));
   s->read_pending[k] = true;

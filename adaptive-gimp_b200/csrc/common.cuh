@@ -18,7 +18,8 @@
 //    the active block list itself.  Active blocks are the 4^d blocks within
 //    one block of any particle's position at that level; every nonzero cell,
 //    node value or node flag of a substep lies inside them.
-//  * particles: SoA, one f32 array per component ([c * N + p]).
+//  * particles: tiles of 32; a tile holds each group of four words of its
+//    particles as 32 consecutive float4 (see Particles).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -71,17 +72,177 @@ struct LevelDev {
   uint32_t* dflag;
 };
 
+// Particle state.  Tiles of 32 particles; a tile is NQ rows of 32 float4, row k
+// holding words 4k .. 4k+3 of its particles.  A warp on consecutive particles
+// reads or writes a row with one 128-bit access per lane (512 contiguous
+// bytes), and all of a particle's words lie at constant offsets from one
+// address (one array per component took an address computation per word).
+// Words a kernel uses together share rows: the binning kernels read row 0,
+// G2P reads the rows before V, P2G all of them.
+//   3D  x y z g | F0..F3 | F4..F7 | F8 m Jp - | vx vy vz C0 | C1..C4 | C5..C8
+//   2D  x y g m | F0..F3 | vx vy C0 C1 | C2 C3 Jp -
+// Integers are stored by their bits.  fl and id are arrays of their own.
 struct Particles {
-  float* x;    // [dim][N]
-  float* v;    // [dim][N]
-  float* F;    // [dim*dim][N]
-  float* C;    // [dim*dim][N]
-  float* m;    // [N]
-  float* Jp;   // [N]
-  int32_t* g;  // [N] prescribed level
+  float4* s;
   int32_t* fl; // [N] level used by the last substep
   int32_t* id; // [N] the particle's index in the caller's arrays
 };
+
+template <int D>
+struct PWord {  // words of a particle
+  static constexpr int X = 0, G = D, F = 4, M = D == 3 ? 13 : 3, JP = 14, V = D == 3 ? 16 : 8, C = V + D;
+  static constexpr int NQ = D == 3 ? 7 : 4;  // rows of a tile
+  static constexpr int PAD = 15;
+};
+
+// float4 of particle p in row 0 of its tile; row k is 32 k further
+template <int D>
+__host__ __device__ __forceinline__ long long prow(long long p) {
+  return (p >> 5) * (PWord<D>::NQ * 32) + (p & 31);
+}
+// word w of particle p (as floats from the state's start)
+template <int D>
+__host__ __device__ __forceinline__ long long pword(long long p, int w) {
+  return (prow<D>(p) + 32 * (w >> 2)) * 4 + (w & 3);
+}
+// float4 of N particles' state
+inline long long state_quads(int dim, long long N) { return (N + 31) / 32 * 32 * (dim == 3 ? 7 : 4); }
+
+// word w of a particle whose rows were loaded into q[]
+__device__ __forceinline__ float qword(const float4* q, int w) {
+  const float4 v = q[w >> 2];
+  return (w & 3) == 0 ? v.x : (w & 3) == 1 ? v.y : (w & 3) == 2 ? v.z : v.w;
+}
+
+// position of particle p
+template <int D>
+__device__ __forceinline__ void load_x(const Particles& P, long long p, float* x) {
+  const float4 v = P.s[prow<D>(p)];
+  x[0] = v.x;
+  x[1] = v.y;
+  if (D == 3) x[2 % D] = v.z;
+}
+
+// Caller arrays of particle fields (particle-major, caller order); null fields
+// are skipped.
+struct Fields {
+  float *x, *v, *F, *C, *m, *Jp;
+  int32_t *g, *fl;
+};
+
+// the caller's array and place of word w of the particle with caller index o;
+// null for fields the caller did not give and for the padding word
+template <int D>
+__device__ __forceinline__ float* field_word(const Fields& f, int w, long long o) {
+  using W = PWord<D>;
+  if (w < D) return f.x ? f.x + o * D + w : nullptr;
+  if (w == W::G) return f.g ? (float*)f.g + o : nullptr;
+  if (w == W::M) return f.m ? f.m + o : nullptr;
+  if (w == W::JP) return f.Jp ? f.Jp + o : nullptr;
+  if (w >= W::F && w < W::F + D * D) return f.F ? f.F + o * (D * D) + (w - W::F) : nullptr;
+  if (w >= W::V && w < W::V + D) return f.v ? f.v + o * D + (w - W::V) : nullptr;
+  if (w >= W::C && w < W::C + D * D) return f.C ? f.C + o * (D * D) + (w - W::C) : nullptr;
+  return nullptr;
+}
+
+// The state of the particle in slot i (caller index o) from the caller's
+// arrays: a row whose fields are all given is one 128-bit store.
+template <int D>
+__device__ __forceinline__ void fields_in(const Particles& P, long long i, const Fields& f, long long o) {
+  float4* q = P.s + prow<D>(i);
+#pragma unroll
+  for (int k = 0; k < PWord<D>::NQ; ++k) {
+    const float* a[4];
+    bool all = true, any = false;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      a[e] = field_word<D>(f, 4 * k + e, o);
+      const bool pad = 4 * k + e == PWord<D>::PAD;
+      all = all && (a[e] || pad);
+      any = any || a[e];
+    }
+    if (all) {
+      q[32 * k] = make_float4(a[0] ? *a[0] : 0.f, a[1] ? *a[1] : 0.f, a[2] ? *a[2] : 0.f, a[3] ? *a[3] : 0.f);
+    } else if (any) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (a[e]) ((float*)(q + 32 * k))[e] = *a[e];
+    }
+  }
+}
+
+// The caller's arrays from the state of a warp's 32 particles, slots
+// [i0, i0 + 32) of n (s: the warp's 32 * FIELD_STRIDE floats).  The caller's
+// order is not the storage order, so each particle's piece of an array lies on
+// its own: pieces of one or a few words are written by their particle's lane,
+// the nine words of a 3D matrix by neighbouring lanes through shared memory
+// (one lane per matrix writes a sector per word: F of 15.5M particles took 634
+// instead of 358 us; for three words the direct form is the faster, 196
+// against 208 us, and so are the loads of fields_in, whose sectors L1 keeps).
+constexpr int FIELD_WARPS = 8;    // warps of a field kernel's CTA
+constexpr int FIELD_STRIDE = 9;   // words per particle in shared memory
+
+__device__ __forceinline__ void matrices_out(const float* m, float* a, float* s, long long o, unsigned live) {
+  const int lane = threadIdx.x & 31;
+  float* const mine = a + o * 9;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s[lane * FIELD_STRIDE + k] = m[k];
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 9; ++r) {
+    const int t = 32 * r + lane, p = t / 9;
+    float* at = (float*)__shfl_sync(0xffffffffu, (unsigned long long)mine, p) + (t - 9 * p);
+    if (live >> p & 1u) *at = s[t];
+  }
+  __syncwarp();
+}
+
+// MAT: the call asks for 3D matrices (F or C).
+template <int D, bool MAT>
+__device__ __forceinline__ void fields_out(const Particles& P, long long i0, long long n, const Fields& f, float* s) {
+  using W = PWord<D>;
+  const long long i = i0 + (threadIdx.x & 31);
+  const bool mine = i < n;
+  const unsigned live = __ballot_sync(0xffffffffu, mine);
+  const long long o = mine ? P.id[i] : 0;
+  const float4* q = P.s + prow<D>(i);
+  Fields direct = f;  // the fields written by the particle's own lane
+  if (MAT) direct.F = direct.C = nullptr;
+  if (mine) {
+#pragma unroll
+    for (int k = 0; k < W::NQ; ++k) {
+      float* a[4];
+      bool any = false;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        a[e] = field_word<D>(direct, 4 * k + e, o);
+        any = any || a[e];
+      }
+      if (!any) continue;
+      const float4 v = __ldg(q + 32 * k);
+      if (a[0]) *a[0] = v.x;
+      if (a[1]) *a[1] = v.y;
+      if (a[2]) *a[2] = v.z;
+      if (a[3]) *a[3] = v.w;
+    }
+    if (f.fl) f.fl[o] = P.fl[i];
+  }
+  if constexpr (MAT) {
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto matrix = [&](int w, float* a) {
+      if (!a) return;
+      float4 v[3];
+      float m[9];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[k] = mine ? __ldg(q + 32 * ((w >> 2) + k)) : zero;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) m[k] = qword(v, (w & 3) + k);
+      matrices_out(m, a, s, o, live);
+    };
+    matrix(W::F, f.F);
+    matrix(W::C, f.C);
+  }
+}
 
 struct Ctx {
   int dim, L, coarsest, sz;
@@ -109,7 +270,7 @@ struct Ctx {
   int32_t* rank_of;
   int32_t* perm;
   int32_t* proj;  // [N] slots of the particles listed for the return map (CTR_PROJ of them)
-  // Particle state, SoA.  P holds the state the substep starts from, in the
+  // Particle state.  P holds the state the substep starts from, in the
   // bin order of the previous substep; G2P writes the new state into Q in this
   // substep's bin order (the host swaps P and Q between substeps).
   Particles P, Q;

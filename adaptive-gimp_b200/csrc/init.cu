@@ -171,6 +171,28 @@ __global__ void __launch_bounds__(1024) k_scan_counts(const int* counts, long lo
   if (threadIdx.x == blockDim.x - 1) offs[n] = part[threadIdx.x];
 }
 
+// particle p's state: F = I, C = 0, Jp = 1, caller index p
+template <int D>
+__device__ __forceinline__ void write_particle(const Particles& P, long long p, const float* x, const float* v, float m,
+                                               int g) {
+  float w[4 * PWord<D>::NQ];
+#pragma unroll
+  for (int k = 0; k < 4 * PWord<D>::NQ; ++k) w[k] = 0.f;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    w[PWord<D>::X + d] = x[d];
+    w[PWord<D>::V + d] = v[d];
+    w[PWord<D>::F + d * (D + 1)] = 1.f;
+  }
+  w[PWord<D>::M] = m;
+  w[PWord<D>::JP] = 1.f;
+  w[PWord<D>::G] = __int_as_float(g);
+#pragma unroll
+  for (int k = 0; k < PWord<D>::NQ; ++k)
+    P.s[prow<D>(p) + 32 * k] = make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]);
+  P.id[p] = (int)p;
+}
+
 template <int D>
 __global__ void __launch_bounds__(TILE) k_lattice_fill(LatticeArgs A, long long ntiles, const long long* offs,
                                                        Particles P, long long N) {
@@ -191,20 +213,10 @@ __global__ void __launch_bounds__(TILE) k_lattice_fill(LatticeArgs A, long long 
     if (in) {
       const long long p = offs[tile] + before + __popc(b & ((1u << lane) - 1u));
       if (p < N) {
+        float xf[D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          P.x[d * N + p] = __double2float_rn(x[d]);
-          P.v[d * N + p] = S.vel[d];
-        }
-#pragma unroll
-        for (int e = 0; e < D * D; ++e) {
-          P.F[e * N + p] = (e % (D + 1) == 0) ? 1.f : 0.f;
-          P.C[e * N + p] = 0.f;
-        }
-        P.m[p] = S.mass;
-        P.Jp[p] = 1.f;
-        P.g[p] = S.level;
-        P.id[p] = (int)p;
+        for (int d = 0; d < D; ++d) xf[d] = __double2float_rn(x[d]);
+        write_particle<D>(P, p, xf, S.vel, S.mass, S.level);
       }
     }
   }
@@ -237,11 +249,9 @@ __global__ void k_random_fill(RandomArgs A, Particles P, long long N) {
     const U4 r = philox(U4{(uint32_t)p, (uint32_t)((unsigned long long)p >> 32), 0u, 0u}, A.k0, A.k1);
     const float u[3] = {u24(r.x), u24(r.y), u24(r.z)};
     // x = u * size + lo in f32 (explicitly rounded: no contraction)
+    float xf[D];
 #pragma unroll
-    for (int d = 0; d < D; ++d) {
-      P.x[d * N + p] = __fadd_rn(__fmul_rn(u[d], B.size[d]), B.lo[d]);
-      P.v[d * N + p] = B.vel[d];
-    }
+    for (int d = 0; d < D; ++d) xf[d] = __fadd_rn(__fmul_rn(u[d], B.size[d]), B.lo[d]);
     int g = B.level;
     for (int k = B.nb - 1; k >= 0; --k) {  // the first matching band wins
       bool in = true;
@@ -249,15 +259,7 @@ __global__ void k_random_fill(RandomArgs A, Particles P, long long N) {
       for (int d = 0; d < D; ++d) in = in && B.blo[k] <= u[d] && u[d] <= B.bhi[k];
       if (in) g = B.blev[k];
     }
-#pragma unroll
-    for (int e = 0; e < D * D; ++e) {
-      P.F[e * N + p] = (e % (D + 1) == 0) ? 1.f : 0.f;
-      P.C[e * N + p] = 0.f;
-    }
-    P.m[p] = B.mass;
-    P.Jp[p] = 1.f;
-    P.g[p] = g;
-    P.id[p] = (int)p;
+    write_particle<D>(P, p, xf, B.vel, B.mass, g);
   }
 }
 

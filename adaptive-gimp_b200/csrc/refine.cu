@@ -33,11 +33,12 @@ __global__ void k_bb_init(Ctx c) {
 template <int D>
 __device__ __forceinline__ bool particle_cell(const Ctx& c, int p, int* cell) {
   bool ok = true;
+  float x[D];
+  load_x<D>(c.P, p, x);
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    const float x = c.P.x[(long long)d * c.N + p];
-    if (!(x >= 0.f && x < 1.f)) ok = false;
-    cell[d] = ok ? (int)floorf(x * (float)c.sz) : 0;
+    if (!(x[d] >= 0.f && x[d] < 1.f)) ok = false;
+    cell[d] = ok ? (int)floorf(x[d] * (float)c.sz) : 0;
   }
   return ok;
 }
@@ -180,7 +181,7 @@ __global__ void k_assign(Ctx c, const uint8_t* depth, int band) {
       break;
     }
   }
-  c.P.g[p] = lv;
+  ((int*)c.P.s)[pword<D>(p, PWord<D>::G)] = lv;
 }
 
 template <int D>

@@ -99,7 +99,9 @@ __global__ void k_render_cells(Ctx c, int res, int show_ghost, int show_node, fl
 __global__ void k_splat(Ctx c, int res, float rpix, int* winner) {
   const long long N = c.N;
   for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < N; s += (long long)gridDim.x * blockDim.x) {
-    const float px = __fmul_rn(c.P.x[s], (float)res), py = __fmul_rn(c.P.x[N + s], (float)res);
+    float x[2];
+    load_x<2>(c.P, s, x);
+    const float px = __fmul_rn(x[0], (float)res), py = __fmul_rn(x[1], (float)res);
     const int id = c.P.id[s];
     const int i0 = max(0, (int)floorf(px - rpix - 0.5f)), i1 = min(res - 1, (int)ceilf(px + rpix - 0.5f));
     const int j0 = max(0, (int)floorf(py - rpix - 0.5f)), j1 = min(res - 1, (int)ceilf(py + rpix - 0.5f));
@@ -179,10 +181,11 @@ __global__ void k_splat3d(Ctx c, agimp_view3d v, int res, const float* dir, unsi
   const float R = v.radius;
   const float fr = (float)res;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < N; i += (long long)gridDim.x * blockDim.x) {
-    float oc[3], w[3];
+    float oc[3], w[3], x[3];
+    load_x<3>(c.P, i, x);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      w[k] = __fsub_rn(c.P.x[k * N + i], v.eye[k]);  // centre relative to the eye
+      w[k] = __fsub_rn(x[k], v.eye[k]);  // centre relative to the eye
       oc[k] = -w[k];
     }
     const float cz = dot3(w, v.forward);
@@ -262,11 +265,12 @@ __global__ void k_shade3d(Ctx c, agimp_view3d v, int res, const float* dir, cons
       shade(v, v.floor_color, hf, n, out);
     } else if (ts < INFINITY) {
       const long long i = slot[(unsigned)(k & 0xffffffffu)];
-      float p[3], n[3];
+      float p[3], n[3], x[3];
+      load_x<3>(c.P, i, x);
 #pragma unroll
       for (int q = 0; q < 3; ++q) {
         p[q] = __fadd_rn(v.eye[q], __fmul_rn(ts, d[q]));
-        n[q] = __fdiv_rn(__fsub_rn(p[q], c.P.x[q * N + i]), v.radius);
+        n[q] = __fdiv_rn(__fsub_rn(p[q], x[q]), v.radius);
       }
       shade(v, v.color, p, n, out);
     }

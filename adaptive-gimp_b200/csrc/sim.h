@@ -105,8 +105,8 @@ struct agimp_batch {
   cudaEvent_t ev_hsrc[2] = {nullptr, nullptr};  // slot k's source table is on the device
   cudaEvent_t ev_gath[2] = {nullptr, nullptr};  // slot k's gather is done
   cudaStream_t gather = nullptr;
-  // batch upload (agimp_batch_set_particles): one field of all scenes in the
-  // staging at a time, the per-scene destinations of all fields in utab
+  // batch upload (agimp_batch_set_particles): one field of all scenes' host
+  // arrays in the staging at a time, the scenes' states in utab
   float* ustage = nullptr;
   size_t ustage_floats = 0;
   void* utab = nullptr;

@@ -122,11 +122,12 @@ __device__ __forceinline__ int grid_init(const Ctx& c, const int* I) {
 template <int D>
 __device__ __forceinline__ void touch_one(const Ctx& c, int p) {
   const bool valid = p < c.N;
+  const float4 row = valid ? c.P.s[prow<D>(p)] : make_float4(0.f, 0.f, 0.f, 0.f);
   float xp[D];
   bool esc = !valid;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    xp[d] = valid ? c.P.x[(long long)d * c.N + p] : 0.f;
+    xp[d] = d == 0 ? row.x : d == 1 ? row.y : row.z;
     if (!(xp[d] >= 0.f && xp[d] < 1.f)) esc = true;
   }
   if (valid && esc) set_err(c, ERR_ESCAPED);
@@ -145,7 +146,7 @@ __device__ __forceinline__ void touch_one(const Ctx& c, int p) {
   // in dynamic mode, L - (level of its level-map cell) in static mode
   unsigned reach = 1;
   if (!c.is_static) {
-    const int gl = c.P.g[p];
+    const int gl = __float_as_int(D == 3 ? row.w : row.z);
     const bool ok = gl >= 0 && gl < c.L;
     int base[D];
     long long bk = ok ? gl : -1;
@@ -595,9 +596,9 @@ __device__ __forceinline__ void bin_one(const Ctx& c, int p, const int* lb) {
   if (p < c.N) {
     float xp[D];
     bool esc = false;
+    load_x<D>(c.P, p, xp);
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      xp[d] = c.P.x[(long long)d * c.N + p];
       if (!(xp[d] >= 0.f && xp[d] < 1.f)) esc = true;
     }
     int fl = -1;

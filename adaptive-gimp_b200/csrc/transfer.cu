@@ -183,22 +183,26 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_p2g(Batch B) {
     int cell = -1;
     if (i < wd.w) {
       const int p = __ldg(&c.perm[wd.z + i]);
-      const long long N = c.N;
       const float inv = (float)(c.coarsest << l);
       const float dx = 1.f / inv;
+      using PW = PWord<D>;
+      float4 st[PW::NQ];
+      const float4* src = c.P.s + prow<D>(p);
+#pragma unroll
+      for (int k = 0; k < PW::NQ; ++k) st[k] = __ldg(src + 32 * k);
       float xp[D], vp[D], F[D * D], Cm[D * D];
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        xp[d] = __ldg(&c.P.x[d * N + p]);
-        vp[d] = __ldg(&c.P.v[d * N + p]);
+        xp[d] = qword(st, PW::X + d);
+        vp[d] = qword(st, PW::V + d);
       }
 #pragma unroll
       for (int k = 0; k < D * D; ++k) {
-        F[k] = __ldg(&c.P.F[k * N + p]);
-        Cm[k] = __ldg(&c.P.C[k * N + p]);
+        F[k] = qword(st, PW::F + k);
+        Cm[k] = qword(st, PW::C + k);
       }
-      const float mp = __ldg(&c.P.m[p]);
-      const float jp = c.plast == 1 ? __ldg(&c.P.Jp[p]) : 1.f;
+      const float mp = qword(st, PW::M);
+      const float jp = qword(st, PW::JP);
       float tc[D];
       cell = 0;
 #pragma unroll
@@ -1095,6 +1099,19 @@ __device__ __forceinline__ void snow_return_map(const Ctx& c, float* F, float& j
   snow_clamp_rebuild<D>(c, U, sg, V, F, jp);
 }
 
+// F and Jp of particle j of a state (the rows' other words stay as they are).
+template <int D>
+__device__ __forceinline__ void store_elastic(const Particles& Q, int j, const float* F, float jp) {
+  using W = PWord<D>;
+  float4* q = Q.s + prow<D>(j);
+  __stwb(q + 32, make_float4(F[0], F[1], F[2], F[3]));
+  if (D == 3) {
+    __stwb(q + 64, make_float4(F[4 % (D * D)], F[5 % (D * D)], F[6 % (D * D)], F[7 % (D * D)]));
+    __stwb((float*)(q + 96), F[D * D - 1]);
+  }
+  __stwb((float*)Q.s + pword<D>(j, W::JP), jp);
+}
+
 // Apply the MLP's predictions: decode the projected singular values sig' and
 // the change of log Jp, reject them when sig' leaves the clamp interval (the
 // yield surface) or the change breaks the plastic-volume balance
@@ -1144,12 +1161,7 @@ __global__ void k_sur_finish(Batch B, const float* __restrict__ meta_all, const 
           F[a * D + b] = acc;
         }
     }
-    const long long N = c.N;
-    float* QF = c.Q.F;
-    float* QJ = c.Q.Jp;
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) __stwb(&QF[k * N + j], F[k]);
-    __stwb(&QJ[j], jp);
+    store_elastic<D>(c.Q, j, F, jp);
   }
 }
 
@@ -1159,50 +1171,98 @@ __global__ void k_sur_finish(Batch B, const float* __restrict__ meta_all, const 
 // level (the extra bin, level -1) are copied unchanged.
 template <int D>
 __device__ __forceinline__ void copy_particle(const Ctx& c, int p, int j) {
-  const long long N = c.N;
+  const float4* src = c.P.s + prow<D>(p);
+  float4* dst = c.Q.s + prow<D>(j);
+#pragma unroll
+  for (int k = 0; k < PWord<D>::NQ; ++k) __stwb(dst + 32 * k, __ldg(src + 32 * k));
+  __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
+  __stwb(&c.Q.fl[j], -1);
+}
+
+// The end of G2P for particle p (slot j of this substep's bin order, level l):
+// the new state from its position, node velocity nv and velocity gradient G
+// (F' = (I + s G) F, whose Gram matrix decides whether the snow return map
+// may change it).  st holds the rows of p before V (x, g, F, m, Jp).
+template <int D>
+__device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, const float4* st, const float* nv,
+                                           const float* G) {
+  using W = PWord<D>;
+  const float pw = (D == 2) ? 0.25f : 0.125f;
+  const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;
+  const float dx = 1.f / (float)(c.coarsest << l);
+  const float s = (c.dt * pw) / (rd * dx);
+  float F[D * D], A[D * D], Fn[D * D], Sg[(D == 2) ? 3 : 6];
+#pragma unroll
+  for (int k = 0; k < D * D; ++k) F[k] = qword(st, W::F + k);
+#pragma unroll
+  for (int i = 0; i < D; ++i)
+#pragma unroll
+    for (int k = 0; k < D; ++k) A[i * D + k] = (i == k ? 1.f : 0.f) + s * G[i * D + k];
+#pragma unroll
+  for (int k = 0; k < ((D == 2) ? 3 : 6); ++k) Sg[k] = 0.f;
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+#pragma unroll
+    for (int q = 0; q < D; ++q) {
+      float a = 0.f;
+#pragma unroll
+      for (int k = 0; k < D; ++k) a += A[i * D + k] * F[k * D + q];
+      Fn[i * D + q] = a;
+    }
+    int u = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+#pragma unroll
+      for (int b = a; b < D; ++b) Sg[u++] += Fn[i * D + a] * Fn[i * D + b];
+  }
+  float w[4 * W::NQ];
+#pragma unroll
+  for (int k = 0; k < 4 * W::NQ; ++k) w[k] = 0.f;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    __stwb(&c.Q.x[d * N + j], __ldg(&c.P.x[d * N + p]));
-    __stwb(&c.Q.v[d * N + j], __ldg(&c.P.v[d * N + p]));
+    w[W::X + d] = qword(st, W::X + d) + c.dt * nv[d];
+    w[W::V + d] = nv[d];
   }
 #pragma unroll
   for (int k = 0; k < D * D; ++k) {
-    __stwb(&c.Q.F[k * N + j], __ldg(&c.P.F[k * N + p]));
-    __stwb(&c.Q.C[k * N + j], __ldg(&c.P.C[k * N + p]));
+    w[W::F + k] = Fn[k];
+    w[W::C + k] = G[k];
   }
-  __stwb(&c.Q.m[j], __ldg(&c.P.m[p]));
-  __stwb(&c.Q.Jp[j], __ldg(&c.P.Jp[p]));
-  __stwb(&c.Q.g[j], __ldg(&c.P.g[p]));
+  w[W::M] = qword(st, W::M);
+  w[W::G] = qword(st, W::G);
+  w[W::JP] = c.plast == 1 ? qword(st, W::JP) : 1.f;
+  float4* dst = c.Q.s + prow<D>(j);
+#pragma unroll
+  for (int k = 0; k < W::NQ; ++k) __stwb(dst + 32 * k, make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
   __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
-  __stwb(&c.Q.fl[j], -1);
+  __stwb(&c.Q.fl[j], l);
+  // trial states that may leave the elastic interval get the return map in
+  // k_project (it needs an SVD, whose registers would halve G2P's occupancy);
+  // det F' = det(I + s G) det F
+  if (c.plast == 1 && !gram_within<D>(Sg, det<D>(A) * det<D>(F), 1.f - c.theta_c, 1.f + c.theta_s))
+    c.proj[reserve_slot(&c.ctr[CTR_PROJ])] = j;
 }
 
 // One particle, slot j of this substep's bin order; the 3^d nodes come
 // through L1 (particles of a bin share a (4+2)^d node tile).
 template <int D>
 __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
-  const float pw = (D == 2) ? 0.25f : 0.125f;
-  const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;
-  const long long N = c.N;
   const int p = __ldg(&c.perm[j]);
   const int l = __ldg(&c.P.fl[p]);
-  // the fields read after the gather start moving into L1 now (no registers held)
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.F[k * N + p]));
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.m[p]));
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.g[p]));
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.id[p]));
-  if (c.plast == 1) asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.Jp[p]));
   if (l < 0) {
     copy_particle<D>(c, p, j);
     return;
   }
+  float4 st[4];  // the rows before V (2D: and the row of Jp)
+  const float4* src = c.P.s + prow<D>(p);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (D == 3 || k != 2) st[k] = __ldg(src + 32 * k);
   float xp[D];
 #pragma unroll
-  for (int d = 0; d < D; ++d) xp[d] = __ldg(&c.P.x[d * N + p]);
+  for (int d = 0; d < D; ++d) xp[d] = qword(st, d);
   const LevelDev& V = c.lev[l];
   const float inv = (float)(c.coarsest << l);
-  const float dx = 1.f / inv;
   int base[D];
   float tc[D];
 #pragma unroll
@@ -1293,58 +1353,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
       }
     }
   }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    __stwb(&c.Q.v[d * N + j], nv[d]);
-    __stwb(&c.Q.x[d * N + j], xp[d] + c.dt * nv[d]);
-  }
-#pragma unroll
-  for (int i = 0; i < D * D; ++i) __stwb(&c.Q.C[i * N + j], G[i]);
-  // the rest of the particle is read only now (fewer live registers during
-  // the gather); m, g, id and Jp travel unchanged
-  __stwb(&c.Q.m[j], __ldg(&c.P.m[p]));
-  __stwb(&c.Q.g[j], __ldg(&c.P.g[p]));
-  __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
-  __stwb(&c.Q.Jp[j], c.plast == 1 ? __ldg(&c.P.Jp[p]) : 1.f);
-  __stwb(&c.Q.fl[j], l);
-  float F[D * D];
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) F[k] = __ldg(&c.P.F[k * N + p]);
-  const float s = (c.dt * pw) / (rd * dx);
-  // F' = (I + s G) F row by row, each row stored at once; the Gram matrix
-  // F'^T F' is summed from the rows for the return-map test below
-  float Sg[(D == 2) ? 3 : 6];
-#pragma unroll
-  for (int k = 0; k < ((D == 2) ? 3 : 6); ++k) Sg[k] = 0.f;
-#pragma unroll
-  for (int i = 0; i < D; ++i) {
-    float row[D];
-#pragma unroll
-    for (int q = 0; q < D; ++q) {
-      float a = 0.f;
-#pragma unroll
-      for (int k = 0; k < D; ++k) a += ((i == k ? 1.f : 0.f) + s * G[i * D + k]) * F[k * D + q];
-      row[q] = a;
-      __stwb(&c.Q.F[(i * D + q) * N + j], a);
-    }
-    int u = 0;
-#pragma unroll
-    for (int a = 0; a < D; ++a)
-#pragma unroll
-      for (int b = a; b < D; ++b) Sg[u++] += row[a] * row[b];
-  }
-  // trial states that may leave the elastic interval get the return map in
-  // k_project (it needs an SVD, whose registers would halve G2P's occupancy);
-  // det F' = det(I + s G) det F
-  if (c.plast == 1) {
-    float A[D * D];
-#pragma unroll
-    for (int i = 0; i < D; ++i)
-#pragma unroll
-      for (int k = 0; k < D; ++k) A[i * D + k] = (i == k ? 1.f : 0.f) + s * G[i * D + k];
-    if (!gram_within<D>(Sg, det<D>(A) * det<D>(F), 1.f - c.theta_c, 1.f + c.theta_s))
-      c.proj[reserve_slot(&c.ctr[CTR_PROJ])] = j;
-  }
+  g2p_finish<D>(c, l, p, j, st, nv, G);
 }
 
 // 2D G2P: one thread per particle slot, grid-stride (a 2D block holds about
@@ -1360,19 +1369,15 @@ __global__ void __launch_bounds__(256, 4) k_g2p_gather(Batch B) {
 // node velocities: txy[t] = (v_x, v_y), tz[t] = v_z of tile node t (the
 // (4+2)^d nodes O..O+5, last axis fastest).
 template <int D>
-__device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, const float* xp, const int* O,
+__device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, const float4* st, const int* O,
                                            const float2* txy, const float* tz) {
-  const float pw = (D == 2) ? 0.25f : 0.125f;
-  const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;
-  const long long N = c.N;
   const float inv = (float)(c.coarsest << l);
-  const float dx = 1.f / inv;
   float tc[D];
   int t0 = 0;
   bool inside = true;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
-    const float xs = xp[d] * inv;
+    const float xs = qword(st, d) * inv;
     const int base = (int)(xs + 0.5f) - 1;
     tc[d] = xs - (float)(base + 1);
     // the binning put the base cell in this block; a cell outside it would
@@ -1457,57 +1462,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
       }
     }
   }
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    __stwb(&c.Q.v[d * N + j], nv[d]);
-    __stwb(&c.Q.x[d * N + j], xp[d] + c.dt * nv[d]);
-  }
-#pragma unroll
-  for (int i = 0; i < D * D; ++i) __stwb(&c.Q.C[i * N + j], G[i]);
-  // m, g, id and Jp travel unchanged
-  __stwb(&c.Q.m[j], __ldg(&c.P.m[p]));
-  __stwb(&c.Q.g[j], __ldg(&c.P.g[p]));
-  __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
-  __stwb(&c.Q.Jp[j], c.plast == 1 ? __ldg(&c.P.Jp[p]) : 1.f);
-  __stwb(&c.Q.fl[j], l);
-  float F[D * D];
-#pragma unroll
-  for (int k = 0; k < D * D; ++k) F[k] = __ldg(&c.P.F[k * N + p]);
-  const float s = (c.dt * pw) / (rd * dx);
-  // F' = (I + s G) F row by row, each row stored at once; the Gram matrix
-  // F'^T F' is summed from the rows for the return-map test below
-  float Sg[(D == 2) ? 3 : 6];
-#pragma unroll
-  for (int k = 0; k < ((D == 2) ? 3 : 6); ++k) Sg[k] = 0.f;
-#pragma unroll
-  for (int i = 0; i < D; ++i) {
-    float row[D];
-#pragma unroll
-    for (int q = 0; q < D; ++q) {
-      float a = 0.f;
-#pragma unroll
-      for (int k = 0; k < D; ++k) a += ((i == k ? 1.f : 0.f) + s * G[i * D + k]) * F[k * D + q];
-      row[q] = a;
-      __stwb(&c.Q.F[(i * D + q) * N + j], a);
-    }
-    int u = 0;
-#pragma unroll
-    for (int a = 0; a < D; ++a)
-#pragma unroll
-      for (int b = a; b < D; ++b) Sg[u++] += row[a] * row[b];
-  }
-  // trial states that may leave the elastic interval get the return map in
-  // k_project (it needs an SVD, whose registers would halve G2P's occupancy);
-  // det F' = det(I + s G) det F
-  if (c.plast == 1) {
-    float A[D * D];
-#pragma unroll
-    for (int i = 0; i < D; ++i)
-#pragma unroll
-      for (int k = 0; k < D; ++k) A[i * D + k] = (i == k ? 1.f : 0.f) + s * G[i * D + k];
-    if (!gram_within<D>(Sg, det<D>(A) * det<D>(F), 1.f - c.theta_c, 1.f + c.theta_s))
-      c.proj[reserve_slot(&c.ctr[CTR_PROJ])] = j;
-  }
+  g2p_finish<D>(c, l, p, j, st, nv, G);
 }
 
 // 3D G2P (adaptive_gimp.py:289-321) over the P2G work items: a CTA takes a
@@ -1526,7 +1481,6 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
   const int nch = c.ctr[CTR_CHUNKS];
   const int per = (nch + nblk_ - 1) / nblk_;
   const int c0 = bid_ * per, c1 = min(nch, c0 + per);
-  const long long N = c.N;
   int tb = 1, tl = -1, tk = -1;
   for (int ch = c0; ch < c1; ++ch) {
     const int4 wd = c.chunks[ch];
@@ -1540,20 +1494,15 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
     const LevelDev& V = c.lev[l];
     int O[D];
     chunk_origin<D>(V, wd.y, O);
-    // the particle's position and the fields read after the gather start
-    // moving before the tile load, so both latencies overlap
+    // the particle's rows before V are requested before the tile load, so both
+    // latencies overlap
     int p = 0;
-    float xp[D];
+    float4 st[4];
     if (mine) {
       p = __ldg(&c.perm[j]);
+      const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
-      for (int d = 0; d < D; ++d) xp[d] = __ldg(&c.P.x[d * N + p]);
-#pragma unroll
-      for (int k = 0; k < D * D; ++k) asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.F[k * N + p]));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.m[p]));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.g[p]));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.id[p]));
-      if (c.plast == 1) asm volatile("prefetch.global.L1 [%0];" ::"l"(&c.P.Jp[p]));
+      for (int k = 0; k < 4; ++k) st[k] = __ldg(src + 32 * k);
     }
     if (l != tl || wd.y != tk) {  // uniform over the CTA
       tb ^= 1;
@@ -1573,7 +1522,7 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
       }
       __syncthreads();
     }
-    if (mine) g2p_staged<D>(c, l, p, j, xp, O, txy[tb], tz[tb]);
+    if (mine) g2p_staged<D>(c, l, p, j, st, O, txy[tb], tz[tb]);
   }
 }
 
@@ -1584,17 +1533,20 @@ __global__ void __launch_bounds__(256) k_project(Batch B) {
   SCENE_CTA(B, MAP_G);
   if (c.plast != 1) return;
   const int n = c.ctr[CTR_PROJ];
-  const long long N = c.N;
+  using W = PWord<D>;
   SCENE_LOOP(s, n) {
     const int j = c.proj[s];
+    const float4* src = c.Q.s + prow<D>(j);
+    float4 st[4];
+#pragma unroll
+    for (int k = 1; k < 4; ++k)
+      if (D == 3 || k != 2) st[k] = src[32 * k];
     float F[D * D];
 #pragma unroll
-    for (int k = 0; k < D * D; ++k) F[k] = c.Q.F[k * N + j];
-    float jp = c.Q.Jp[j];
+    for (int k = 0; k < D * D; ++k) F[k] = qword(st, W::F + k);
+    float jp = qword(st, W::JP);
     snow_return_map<D>(c, F, jp, j);
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) __stwb(&c.Q.F[k * N + j], F[k]);
-    __stwb(&c.Q.Jp[j], jp);
+    store_elastic<D>(c.Q, j, F, jp);
   }
 }
 
