@@ -519,6 +519,46 @@ __device__ __forceinline__ long long total_elems(const Ctx& c, int l0, int l1, i
   return t << (2 * D);
 }
 
+#ifdef __CUDACC__
+// ---------------------------------------------------------------------------
+// Packed f32x2 arithmetic (sm_100 fma/mul/add .f32x2): each half is rounded
+// exactly like the scalar fmaf / multiply / add, at one instruction per pair.
+// f2: a pair in a 64-bit register.
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_dup(float a) { return f2_make(a, a); }
+__device__ __forceinline__ float2 f2_get(f2 r) {
+  float2 a;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
+  return a;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+// the same on float2 operands
+__device__ __forceinline__ f2 pk2(float2 a) { return f2_make(a.x, a.y); }
+__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return f2_get(f2_fma(pk2(a), pk2(b), pk2(c))); }
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return f2_get(f2_mul(pk2(a), pk2(b))); }
+__device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return f2_get(f2_add(pk2(a), pk2(b))); }
+__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
+#endif
+
 // ---------------------------------------------------------------------------
 // small dense linear algebra (row-major)
 template <int D>

@@ -39,36 +39,6 @@ __device__ __forceinline__ void chunk_origin(const LevelDev& V, long long blk, i
 }
 
 // ---------------------------------------------------------------------------
-// Packed f32x2 arithmetic (sm_100 fma/mul/add .f32x2): each half is rounded
-// exactly like the scalar fmaf / multiply / add, at one instruction per pair.
-__device__ __forceinline__ unsigned long long pk2(float2 a) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
-  return r;
-}
-__device__ __forceinline__ float2 upk2(unsigned long long r) {
-  float2 a;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a.x), "=f"(a.y) : "l"(r));
-  return a;
-}
-__device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)), "l"(pk2(c)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
-  unsigned long long d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pk2(a)), "l"(pk2(b)));
-  return upk2(d);
-}
-__device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
-
-// ---------------------------------------------------------------------------
 // P2G (adaptive_gimp.py:230-250).  Per work item (up to CH particles of one
 // 4^d block of one level, in base-cell order: bins store their particles
 // sorted by cell, the last axis fastest):
