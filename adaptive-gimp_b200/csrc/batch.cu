@@ -168,11 +168,10 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
   long long sumN = 0;
   for (agimp_sim* s : b->sims) sumN += s->c.N;
   const long long G = (long long)b->sms * b->tune.ctas_per_sm;
-  // P2G: whole waves of resident CTAs (a partly filled last wave leaves SMs
-  // idle at the end of the kernel), at least as many CTAs as the other kinds
-  const int res = p2g_resident(b->dim, b->tune.chunk);
-  const long long wave = (long long)b->sms * res;
-  const long long GP = std::max<long long>(1, (G + wave - 1) / wave) * wave;
+  // P2G: one wave of resident CTAs for a single scene (a warp takes an equal
+  // range of the work items; with more waves a small scene's few items would
+  // wait for one another), four for a batch (the scenes' shares are whole CTAs)
+  const long long GP = (long long)b->sms * p2g_resident(b->dim) * (n == 1 ? 1 : 4);
   int* Gm = b->hofs.data() + MAP_G * (n + 1);
   int* O = b->hofs.data() + MAP_O * (n + 1);
   int* T = b->hofs.data() + MAP_T * (n + 1);
@@ -587,7 +586,7 @@ agimp_status batch_set_tuning(agimp_batch* b, const agimp_tuning* t) {
 }
 
 // ---------------------------------------------------------------------------
-// Autotuner.  Every candidate (P2G work-item size x grid-stride CTAs per SM)
+// Autotuner.  Every candidate (G2P work-item size x grid-stride CTAs per SM)
 // runs `trials` timed substeps after two warm-up substeps (which capture its
 // graphs) from the same saved particle state; the fastest is kept.  The saved
 // state is put back after each candidate, so tuning leaves the simulation

@@ -400,6 +400,8 @@ agimp_status agimp_create(const agimp_params* p, int32_t device, agimp_sim** out
   cudaMemset(c.cell_count, 0, (tot_blocks + 1) * per * sizeof(int32_t));
   const long long N = c.N;
   AL(c.chunks, N / MIN_CHUNK + tot_blocks + 2);  // enough for any work-item size
+  // a bin's items: its tasks over P2G_TASKS, rounded up; at most one task per particle
+  AL(c.items, N / P2G_TASKS + std::min<long long>(N, tot_blocks) + 2);
   c.chunk = CHUNK;
   AL(c.bin_of, N + 1);
   AL(c.rank_of, N + 1);

@@ -27,10 +27,19 @@
 namespace agimp {
 
 constexpr int MAXL = 8;
-constexpr int CHUNK = 256;      // default P2G work item (particles of one bin) = P2G CTA size
+constexpr int CHUNK = 256;      // default G2P work item (particles of one bin) = 3D G2P CTA size
 constexpr int MAX_CHUNK = 512;  // largest work item the tuning may choose
 constexpr int MIN_CHUNK = 64;   // smallest work item (sizes the work-item buffer)
 constexpr int HALO = 4;
+
+// P2G work items (k_p2g): up to P2G_TASKS tasks of up to T = 2^p2g_log_task
+// particles of one base cell; T is chosen per bin from its particles per
+// non-empty cell and the scene's size (small scenes have more warps than items:
+// shorter tasks make more of them).
+constexpr int P2G_TASKS = 10, P2G_LOG_TMAX = 3;
+__host__ __device__ constexpr int p2g_log_task(int per_cell, int n) {
+  return per_cell <= 4 || n < 150000 ? 2 : P2G_LOG_TMAX;
+}
 
 enum : uint32_t { ACT = 1u, GHO = 2u, TJ = 4u, CUL = 8u };
 enum : uint32_t { ERR_OOB = 1u, ERR_ESCAPED = 2u, ERR_MAP_OOB = 4u, ERR_NOBIN = 8u, ERR_MLP = 16u };
@@ -40,7 +49,7 @@ enum {
   CTR_LEVEL = 0,   // [0, MAXL): active blocks per level
   CTR_TOUCH = 8,   // touched finest blocks
   CTR_BINCUR = 9,  // particles placed by the bin allocator
-  CTR_CHUNKS = 10, // P2G/G2P work items
+  CTR_CHUNKS = 10, // G2P work items
   CTR_ERR = 11,    // error bits
   CTR_UNBIN = 12,  // particles without a level (fl_p = -1) in the last substep
   CTR_SUR = 13,    // particles handed to the surrogate MLP in the last substep
@@ -49,7 +58,8 @@ enum {
   // [16, 22): particle bounding box used by the refinement rule
   CTR_PROJ = 22,   // particles whose trial state needs the return map this substep
   CTR_FULL = 23,   // non-empty bins this substep (listed in full_bins)
-  CTR_COUNT = 24
+  CTR_ITEMS = 24,  // P2G work items this substep
+  CTR_COUNT = 25
 };
 
 struct LevelDev {
@@ -250,7 +260,7 @@ struct Ctx {
   int sms;  // multiprocessors of the device (grid-stride launch width)
   int is_static, gap, bmode, plast, ncol, map_h, map_n;
   int inv_norm;  // 1: normalise nodes that are not activated (extension)
-  int chunk;     // particles per P2G work item: 64, 128 or 256 (launch tuning)
+  int chunk;     // particles per 3D G2P work item: 64, 128, 256 or 512 (launch tuning)
   float radius, mu, la, theta_c, theta_s, xi, dt;
   float grav[3];
   double col[4][6];  // collider boxes, compared in double like the oracle
@@ -266,6 +276,7 @@ struct Ctx {
   int32_t* bin_start;
   int32_t* full_bins;   // [bins]: the non-empty bins of this substep
   int4* chunks;  // {level, block (stored linear id), start, count}
+  int4* items;   // P2G: {level | log2 T << 4 | item of the bin << 8, block (stored linear id), bin, particles of the bin}
   int32_t* bin_of;      // per particle: bin * 4^d + base cell
   int32_t* rank_of;
   int32_t* perm;
@@ -1037,7 +1048,7 @@ __host__ __device__ __forceinline__ void axis_weights_half(float t, float* W, fl
 enum { MAP_G = 0,  // grid-stride kernels over particles, active blocks or work items
        MAP_O = 1,  // bin allocation (1024-thread CTAs)
        MAP_T = 2,  // staged level transfers (one 4^d block per CTA at a time: 4x MAP_G's CTAs)
-       MAP_P = 3,  // P2G: whole waves of the CTAs that fit an SM at once
+       MAP_P = 3,  // P2G: one wave (batches: four) of the CTAs that fit the SMs at once
        NMAP = 4 };
 
 struct Batch {
@@ -1053,7 +1064,7 @@ struct BatchLaunch {
   int sms;           // multiprocessors of the device
   int maxL;          // most levels of any scene (per-level launches run to it)
   int nct[NMAP];     // CTAs of each launch kind
-  int chunk;         // P2G work-item size of every scene
+  int chunk;         // 3D G2P work-item size of every scene
   int any_dynamic;   // some scene activates cells from g_p (runs k_mark_hier)
   int any_plastic;   // some scene has snow plasticity (runs k_project)
   const Ctx* single; // host context of a single simulator, else null
@@ -1156,7 +1167,7 @@ constexpr int PHASES = 8;  // blocks, topology, binning, p2g, restrict, gridop, 
 void launch_substep(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev = nullptr);
 void launch_refine(const Ctx& c, int band, cudaStream_t s);
 void prepare_transfer_kernels();  // kernel attributes (shared-memory opt-in); once per device
-int p2g_resident(int dim, int chunk);  // k_p2g CTAs an SM holds at once
+int p2g_resident(int dim);  // k_p2g CTAs an SM holds at once
 // surrogate MLP forward over a device-side sample count (mlp.cu)
 void launch_mlp_forward_dev(const void* packed, const float* P, const float* X, float* Y, const int32_t* n_dev,
                             long long cap, int32_t* err, int sms, cudaStream_t s);

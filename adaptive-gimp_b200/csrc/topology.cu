@@ -53,6 +53,7 @@ __global__ void k_clear(Batch B) {
     if (c.sur) *c.sur_ctr = 0;  // a batch's shared slot counter (every scene clears it)
     c.ctr[CTR_PROJ] = 0;
     c.ctr[CTR_FULL] = 0;
+    c.ctr[CTR_ITEMS] = 0;
   }
   __shared__ BlockRanges br;
   load_block_ranges(c, br);
@@ -762,7 +763,9 @@ __global__ void __launch_bounds__(1024) k_offsets(Batch B) {
 }
 
 // Offsets of the cells inside each bin (the bin's particles are stored in
-// cell order); one warp per bin, cell counts cleared for the next substep.
+// cell order) and the bin's P2G work items (up to P2G_TASKS tasks of up to
+// 2^p2g_log_task particles of one cell each); one warp per bin, cell counts cleared for the
+// next substep.
 template <int D>
 __global__ void k_cell_offsets(Batch B) {
   SCENE_CTA(B, MAP_G);
@@ -770,15 +773,18 @@ __global__ void k_cell_offsets(Batch B) {
   const int lane = threadIdx.x & 31;
   const int wid = bid_ * (blockDim.x >> 5) + (threadIdx.x >> 5), nw = nblk_ * (blockDim.x >> 5);
   const int nfull = c.ctr[CTR_FULL];
+  int nblk = 0;
+  for (int q = 0; q < c.L; ++q) nblk += c.ctr[CTR_LEVEL + q];
   for (int t = wid; t < nfull; t += nw) {
     const int b = c.full_bins[t];
     int* cc = c.cell_count + ((long long)b << (2 * D));
-    int n[PER], tot = 0;
+    int n[PER], tot = 0, used = 0;
 #pragma unroll
     for (int k = 0; k < PER; ++k) {
       const int cell = lane * PER + k;
       n[k] = cell < NC ? cc[cell] : 0;
       tot += n[k];
+      used += n[k] > 0;
     }
     int inc = tot;  // inclusive scan of the lanes' totals
 #pragma unroll
@@ -797,6 +803,24 @@ __global__ void k_cell_offsets(Batch B) {
         if (n[k]) cc[cell] = 0;
       }
     }
+    if (b >= nblk) continue;  // the bin of particles without a level: no transfer
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const int lt = p2g_log_task(total / __reduce_add_sync(0xffffffffu, used), c.N);
+    int tasks = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) tasks += (n[k] + (1 << lt) - 1) >> lt;
+    tasks = __reduce_add_sync(0xffffffffu, tasks);
+    const int ni = (tasks + P2G_TASKS - 1) / P2G_TASKS;
+    int i0 = 0;
+    if (lane == 0) i0 = atomicAdd(&c.ctr[CTR_ITEMS], ni);
+    i0 = __shfl_sync(0xffffffffu, i0, 0);
+    int l = 0, r = b;
+    while (l < c.L - 1 && r >= c.ctr[CTR_LEVEL + l]) {
+      r -= c.ctr[CTR_LEVEL + l];
+      ++l;
+    }
+    const int blk = c.lev[l].blist[r];
+    for (int k = lane; k < ni; k += 32) c.items[i0 + k] = make_int4(l | (lt << 4) | (k << 8), blk, b, total);
   }
 }
 

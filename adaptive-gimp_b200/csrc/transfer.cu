@@ -9,11 +9,12 @@
 //   303-321 grid_prolongation -> k_prolong  (one launch per level, coarse->fine)
 //   252-275 g2p               -> k_g2p      (all levels in one launch)
 //
-// P2G: one CTA per work item = up to CH particles of one bin (one 4^d block of
-// one level).  A bin's particles touch only the (4+2)^d nodes from the block
-// origin, so P2G accumulates into that tile in shared memory and flushes it
-// with one float4 atomic per touched node.  G2P: one thread per particle slot
-// in bin order; neighbouring threads gather the same nodes through L1.
+// P2G: one warp per work item = some tens of particles of one bin (one 4^d
+// block of one level).  A bin's particles touch only the (4+2)^d nodes from the
+// block origin, so P2G accumulates into that tile in shared memory and flushes
+// it with one float4 atomic per touched node.  G2P: one thread per particle
+// slot in bin order; 3D reads the nodes from a tile staged per block, 2D
+// gathers them through L1.
 //
 // Every kernel serves a batch of scenes (a single simulator is a batch of
 // one): each CTA works for the scene its launch range assigns it to.
@@ -39,370 +40,439 @@ __device__ __forceinline__ void chunk_origin(const LevelDev& V, long long blk, i
 }
 
 // ---------------------------------------------------------------------------
-// P2G (adaptive_gimp.py:230-250).  Per work item (up to CH particles of one
-// 4^d block of one level, in base-cell order: bins store their particles
-// sorted by cell, the last axis fastest):
-//  1. one thread per particle computes the scaled Kirchhoff stress S
-//     (utils.py:11-16, adaptive_gimp.py:240; symmetric, kirchhoff_sym), its
-//     per-axis GIMP weights and gradients, m, a = m (v - C (tc+1)) and
-//     B = m C, and its base cell inside the block, forms each node row's
-//     share A of the momentum term (below) and stores the record in shared
-//     memory at its thread index;
-//  2. each warp cuts its own 32 particles into ranges: in 3D SLOTS = 3
-//     contiguous ranges of equal length (11/11/10), which keeps every slot
-//     busy for the same number of steps; in 2D runs of one base cell (about 4
-//     particles), 10 at a time.  A lane owns one row of three
-//     stencil nodes (the last axis runs along the row; 3^(d-1) rows per cell)
-//     of one range and walks its particles, reading its row's float4 and the
-//     record's shared part (3D 18 floats, 2D 16, of 52 / 28).  It sums the
-//     three nodes' w m and w (a + B n) + S grad w in registers; when the base
-//     cell moves one or two cells along the row, the nodes left behind go to
-//     the (4+2)^d node tile in shared memory and the others move down the
-//     row; any other change, and the end, sends all three;
-//  3. a CTA takes a contiguous range of work items, so consecutive items of
-//     one block (a dense block holds many) keep summing into the same tile;
-//     when the next item is another block, the tile is flushed after one
-//     barrier with one float4 atomic per touched node and cleared.  Two tiles
-//     alternate between blocks, so the next block's records and sums need no
-//     further barrier.
-template <int D, int CH>
+// P2G (adaptive_gimp.py:230-250).  Each warp works alone on a contiguous range
+// of work items (k_cell_offsets): an item is up to TASKS tasks of one 4^d block
+// of one level, a task up to T particles of one base cell (bins store their
+// particles sorted by cell, so an item's particles are contiguous).
+//  1. Rounds of 32 particles, one per lane: the scaled Kirchhoff stress S
+//     (utils.py:11-16, adaptive_gimp.py:240; symmetric, kirchhoff_sym), m,
+//     a = m (v - C (tc+1)), B = m C and tc go to shared memory, at [place in
+//     its task][task].
+//  2. The tasks' contributions to their cell's 3^d nodes are summed in registers
+//     (packed f32x2), by three lanes per task, one per plane (3D) or row (2D) of
+//     nodes along the first axis: all 27 nodes' sums in one lane leave room for
+//     8 warps on an SM (200 instead of 132 us for 1.9M particles), and in 2D
+//     the three lanes make a small scene's items shorter.
+//  3. The sums go through shared memory to one lane per node, which adds the
+//     tasks of one cell and updates the warp's (4+2)^d node tile.
+// The tile goes to the grid with one float4 atomic per touched node when the
+// warp's next item is another block.  There are no atomics on shared memory
+// (an f32 add there is a compare-and-swap loop) and no CTA barriers.
+//
+// What bounds it: instruction issue (38 warp instructions per 3D particle, half
+// of them multiply-adds, at 52 percent of the issue slots) and, between, the
+// latency of step 1's reads at 16 warps per SM.  Before (one lane per row of
+// three nodes, a 52-float record read by nine lanes, shared-memory atomics at
+// every change of cell) it took 53.  1.9M 3D particles on three levels 172 ->
+// 129 us, 15.5M 1210 -> 900, 0.6M at 8 per cell 70 -> 53, 50,000 16.6 -> 11.3;
+// 4.1M 2D particles at 4 per cell 254 (at the best of its CTA sizes, 613 at the
+// default) -> 213 us.  Also measured: long tasks in dense cells (up to 32
+// particles: 273 us, a warp's range of items then differs in cost), the next
+// round's rows in registers (152: spills), 5 CTAs of 96 registers (176).
+template <int D>
 struct P2GLayout {
-  static constexpr int ROWS = (D == 2) ? 3 : 9;   // node rows per stencil
-  static constexpr int SLOTS = 32 / ROWS;         // particle ranges served by one warp at once
+  static constexpr int WARPS = 4;                 // warps of a CTA
+  static constexpr int CTAS = D == 2 ? 8 : 4;     // CTAs an SM should hold
+  static constexpr int NN = (D == 2) ? 9 : 27;    // stencil nodes
+  static constexpr int SPLIT = 3;                 // lanes of a task
+  static constexpr int PN = NN / SPLIT;           // their nodes
   static constexpr int TN = (D == 2) ? 36 : 216;  // nodes of the (4+2)^d tile
-  // per-particle record (floats): one float4 per node row (a lane reads only
-  // its own row and the part every row shares):
-  //  3D  4 r: A_x A_y A_z cw of row r = 3 n0 + n1 (r < 9) | 36 Bk_x Bk_y Bk_z m |
-  //     40 SL_x SL_y SL_z cell | 44 W2[0..2] G2[0] | 48 G2[1] G2[2] - -
-  //  2D  4 r: A_x A_y cw cell of row r = n0 (r < 3) | 12 Bk_x Bk_y SL_x SL_y |
-  //     16 W1[0..2] m | 20 G1[0..2] - | 24 - - - -
-  // Strides are odd multiples of four floats: the float4 stores of eight
-  // consecutive threads (one shared-memory wavefront) fall in distinct banks.
-  static constexpr int STRIDE = (D == 3) ? 52 : 28;
-  static constexpr int TMAX = 16;  // 2D: longest run of one base cell walked by one slot
-  static constexpr size_t bytes() {
-    return sizeof(float) * ((size_t)CH * STRIDE + 2 * 4 * TN) + sizeof(int) * (CH / 32) * 33;
-  }
+  static constexpr int TASKS = P2G_TASKS, TMAX = 1 << P2G_LOG_TMAX;
+  // step 3: groups of node lanes, each with its share of the tasks and its own
+  // tile (3D 27 lanes, 2D 3 x 9 lanes)
+  static constexpr int GROUPS = 32 / NN;
+  // record (floats): 3D  0 a m | 4 B0 t0 | 8 B1 t1 | 12 B2 t2 | 16 Sxx Sxy Sxz Syz | 20 Syy Szz
+  //                  2D  0 a m t0 | 4 B0 B1 | 8 Sxx Sxy Syy t1
+  // (B_d: column d of m C).  REC and ROW put the float4 accesses of eight
+  // neighbouring lanes in distinct banks, by task (step 2) and by place (step
+  // 1, where consecutive particles are consecutive places of a task).
+  static constexpr int REC = (D == 2) ? 12 : 28;
+  static constexpr int ROW = TASKS * REC + (D == 2 ? 12 : 4);
+  static constexpr int RECS = TMAX * ROW, SUMS = TASKS * NN * 4;  // records, then the lanes' sums
+  static constexpr int AREA = RECS > SUMS ? RECS : SUMS;
+  static constexpr int WARP_FLOATS = AREA + GROUPS * TN * 4;
+  static constexpr size_t bytes() { return sizeof(float) * (size_t)WARPS * WARP_FLOATS; }
 };
 
-// Node k of a lane's row of base cell cc sits at tile index row_tile + k.
+// Step 1: the record of particle p of a level (inv = 1 / dx) at R.  The stress
+// carries sc = 2 (-dt 0.5^d) / (radius^d dx): the factor kg / kw = 2 of the
+// gradient weights; the sums get kw when they leave the tile.
 template <int D>
-__device__ __forceinline__ int p2g_row_tile(int cc, int n0, int n1) {
-  if (D == 2) return (((cc >> 2) & 3) + n0) * 6 + (cc & 3);
-  return ((((cc >> 4) & 3) + n0) * 6 + ((cc >> 2) & 3) + n1) * 6 + (cc & 3);
-}
-
-// One node's sums into the node tile ([4][TN]: p_x, p_y, p_z, m).
-template <int D>
-__device__ __forceinline__ void p2g_node_flush(float* tile, int TN, int ti, float2 axy, float az, float am) {
-  atomicAdd(&tile[ti], axy.x);
-  atomicAdd(&tile[TN + ti], axy.y);
-  if (D == 3) atomicAdd(&tile[2 * TN + ti], az);
-  atomicAdd(&tile[3 * TN + ti], am);
-}
-
-// A lane's three node sums of one base cell into the node tile.
-template <int D>
-__device__ __forceinline__ void p2g_row_flush(float* tile, int TN, int cc, int n0, int n1, const float2* axy,
-                                              const float* az, const float* am) {
-  const int ti = p2g_row_tile<D>(cc, n0, n1);
+__device__ __forceinline__ void p2g_record(const Ctx& c, int p, float inv, float sc, float* R) {
+  using W = PWord<D>;
+  float4 q[W::NQ];
+  const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) p2g_node_flush<D>(tile, TN, ti + k, axy[k], az[k], am[k]);
+  for (int k = 0; k < W::NQ; ++k) q[k] = __ldg(src + 32 * k);
+  float t[D], F[D * D];
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    const float xs = qword(q, W::X + d) * inv;
+    const int base = (int)(xs + 0.5f) - 1;
+    t[d] = xs - (float)(base + 1);
+  }
+#pragma unroll
+  for (int k = 0; k < D * D; ++k) F[k] = qword(q, W::F + k);
+  const float m = qword(q, W::M);
+  float mu = c.mu, la = c.la;
+  if (c.plast == 1) {
+    const float h = expf(c.xi * (1.f - qword(q, W::JP)));
+    mu *= h;
+    la *= h;
+  }
+  const float J = det<D>(F);
+  float S[(D == 2) ? 3 : 6];
+  kirchhoff_sym<D>(F, 2.f * mu, la * J * (J - 1.f), S);
+  float a[D];
+#pragma unroll
+  for (int i = 0; i < D; ++i) {
+    float cd = 0.f;
+#pragma unroll
+    for (int b = 0; b < D; ++b) cd += qword(q, W::C + i * D + b) * (t[b] + 1.f);
+    a[i] = m * (qword(q, W::V + i) - cd);
+  }
+  auto B = [&](int i, int d) { return m * qword(q, W::C + i * D + d); };
+  float4* R4 = (float4*)R;
+  if constexpr (D == 3) {
+    R4[0] = make_float4(a[0], a[1], a[2], m);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) R4[1 + d] = make_float4(B(0, d), B(1, d), B(2, d), t[d]);
+    R4[4] = make_float4(sc * S[0], sc * S[1], sc * S[3], sc * S[4]);
+    *(float2*)(R4 + 5) = make_float2(sc * S[2], sc * S[5]);
+  } else {
+    R4[0] = make_float4(a[0], a[1], m, t[0]);
+    R4[1] = make_float4(B(0, 0), B(1, 0), B(0, 1), B(1, 1));
+    R4[2] = make_float4(sc * S[0], sc * S[1], sc * S[2], t[1]);
+  }
 }
 
-template <int D, int CH>
-__global__ void __launch_bounds__(CH, 1024 / CH) k_p2g(Batch B) {
-  SCENE_CTA(B, MAP_P);
-  using Y = P2GLayout<D, CH>;
-  extern __shared__ float4 dsm4[];
-  float* pd = (float*)dsm4;             // [CH][STRIDE]
-  float* tiles = pd + CH * Y::STRIDE;   // [2][4][TN]: p_x, p_y, p_z, m
-  int* starts = (int*)(tiles + 2 * 4 * Y::TN);  // 2D: [warps][33] run starts
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nch = c.ctr[CTR_CHUNKS];
-  const float pw = (D == 2) ? 0.25f : 0.125f;                                        // 0.5**dim
-  const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;  // radius**dim
-  const float r2 = 2.f * c.radius;
-  const float kw = (D == 2) ? 1.f / (4.f * r2 * r2) : 1.f / (8.f * r2 * r2 * r2);
-  const bool half = c.radius == 0.5f;
-  // the tiles start at zero; each flush leaves its tile at zero again
-  for (int i = threadIdx.x; i < 2 * 4 * Y::TN; i += blockDim.x) tiles[i] = 0.f;
-  __syncthreads();
-  int tb = 0;
-  const int per = (nch + nblk_ - 1) / nblk_;
-  const int c0 = bid_ * per, c1 = min(nch, c0 + per);
-  // this lane's slot and node row
-  const int q = lane / Y::ROWS, row = lane % Y::ROWS;
-  const int n0 = (D == 2) ? row : row / 3, n1 = (D == 2) ? 0 : row % 3;
-  for (int ch = c0; ch < c1; ++ch) {
-    const int4 wd = c.chunks[ch];
-    const int l = wd.x;
-    if (l < 0) continue;  // particles without a level: no transfer (uniform over the CTA)
-    // the tile is flushed when the next work item of this CTA is another block
-    bool last = ch + 1 == c1;
-    if (!last) {
-      const int4 nx = c.chunks[ch + 1];
-      last = nx.x != wd.x || nx.y != wd.y;
+// One axis's weights and gradients, each twice (packed operands); for radius
+// 1/2 axis_weights_half's closed form.
+__device__ __forceinline__ void p2g_axis(float t, float radius, bool half, f2* w, f2* g) {
+  if (half) {
+    const f2 t2 = f2_dup(t);
+    g[0] = f2_add(t2, f2_dup(-0.5f));
+    g[1] = f2_mul(t2, f2_dup(-2.f));
+    g[2] = f2_add(t2, f2_dup(0.5f));
+    w[0] = f2_mul(g[0], g[0]);
+    w[1] = f2_fma(g[1], t2, f2_dup(1.5f));
+    w[2] = f2_mul(g[2], g[2]);
+  } else {
+    float W[3], G[3];
+    axis_weights(t, radius, W, G);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      w[k] = f2_dup(W[k]);
+      g[k] = f2_dup(G[k]);
     }
+  }
+}
+
+// Weight and gradient of node n0 of the first axis: for radius 1/2, with q = t
+// + (n0 - 1) / 2, the gradient is b q and the weight b q^2 + e, (b, e) = (1, 0),
+// (-2, 3/2), (1, 0).
+__device__ __forceinline__ void p2g_axis_at(float t, float radius, bool half, int n0, f2& w, f2& g) {
+  if (half) {
+    const float q = t + 0.5f * (float)(n0 - 1);
+    const float gs = n0 == 1 ? -2.f * q : q;
+    g = f2_dup(gs);
+    w = f2_dup(fmaf(gs, q, n0 == 1 ? 1.5f : 0.f));
+  } else {
+    float W[3], G[3];
+    axis_weights(t, radius, W, G);
+    g = f2_dup(n0 == 0 ? G[0] : n0 == 1 ? G[1] : G[2]);
+    w = f2_dup(n0 == 0 ? W[0] : n0 == 1 ? W[1] : W[2]);
+  }
+}
+
+// Step 2: one particle into the sums of plane n0.  A node's term (unscaled, see
+// p2g_record) is
+//   w (a + B n) + S grad w = Wz (A + k Bz') + Gz Sz',
+//   A = Wy (P + n1 Wx By) + Gy Wx Sy,  P = Wx (a + n0 Bx) + Gx Sx,
+//   Bz' = Wx Wy Bz,  Sz' = Wx Wy Sz   (B_d, S_d: columns)
+// 3D node n = 3 n1 + k: xy[n] = (p_x, p_y), zm[n] = (p_z, m): the mass rides as
+// the fourth component of a (B and S have none).
+__device__ __forceinline__ void p2g_plane(const float* R, float radius, bool half, int n0, f2* xy, f2* zm) {
+  const float4* R4 = (const float4*)R;
+  const float4 a = R4[0], b0 = R4[1], b1 = R4[2], b2 = R4[3], s = R4[4];
+  const float2 e = *(const float2*)(R4 + 5);  // Syy Szz
+  f2 wx, gx, wy[3], gy[3], wz[3], gz[3];
+  p2g_axis_at(b0.w, radius, half, n0, wx, gx);
+  p2g_axis(b1.w, radius, half, wy, gy);
+  p2g_axis(b2.w, radius, half, wz, gz);
+  const f2 fn = f2_dup((float)n0);
+  const f2 u = f2_fma(fn, f2_make(b0.x, b0.y), f2_make(a.x, a.y));
+  const f2 z = f2_fma(fn, f2_make(b0.z, 0.f), f2_make(a.z, a.w));
+  f2 P = f2_fma(wx, u, f2_mul(gx, f2_make(s.x, s.y))), Pz = f2_fma(wx, z, f2_mul(gx, f2_make(s.z, 0.f)));
+  const f2 Q = f2_mul(wx, f2_make(b1.x, b1.y)), Qz = f2_mul(wx, f2_make(b1.z, 0.f));
+  const f2 T = f2_mul(wx, f2_make(s.y, e.x)), Tz = f2_mul(wx, f2_make(s.w, 0.f));
+  const f2 E = f2_mul(wx, f2_make(b2.x, b2.y)), Ez = f2_mul(wx, f2_make(b2.z, 0.f));
+  const f2 H = f2_mul(wx, f2_make(s.z, s.w)), Hz = f2_mul(wx, f2_make(e.y, 0.f));
+#pragma unroll
+  for (int n1 = 0; n1 < 3; ++n1) {
+    f2 A = f2_fma(wy[n1], P, f2_mul(gy[n1], T)), Az = f2_fma(wy[n1], Pz, f2_mul(gy[n1], Tz));
+    const f2 b = f2_mul(wy[n1], E), bz = f2_mul(wy[n1], Ez), h = f2_mul(wy[n1], H), hz = f2_mul(wy[n1], Hz);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      xy[3 * n1 + k] = f2_fma(gz[k], h, f2_fma(wz[k], A, xy[3 * n1 + k]));
+      zm[3 * n1 + k] = f2_fma(gz[k], hz, f2_fma(wz[k], Az, zm[3 * n1 + k]));
+      if (k < 2) {
+        A = f2_add(A, b);
+        Az = f2_add(Az, bz);
+      }
+    }
+    if (n1 < 2) {
+      P = f2_add(P, Q);
+      Pz = f2_add(Pz, Qz);
+    }
+  }
+}
+
+// 2D row n0: xy[k] = (p_x, p_y), m[k].
+__device__ __forceinline__ void p2g_row(const float* R, float radius, bool half, int n0, f2* xy, float* m) {
+  const float4* R4 = (const float4*)R;
+  const float4 a = R4[0], b = R4[1], s = R4[2];
+  f2 wx, gx, wy[3], gy[3];
+  p2g_axis_at(a.w, radius, half, n0, wx, gx);
+  p2g_axis(s.w, radius, half, wy, gy);
+  const f2 u = f2_fma(f2_dup((float)n0), f2_make(b.x, b.y), f2_make(a.x, a.y));
+  f2 A = f2_fma(wx, u, f2_mul(gx, f2_make(s.x, s.y)));
+  const f2 e = f2_mul(wx, f2_make(b.z, b.w)), h = f2_mul(wx, f2_make(s.y, s.z));
+  const float cm = f2_get(wx).x * a.z;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    xy[k] = f2_fma(gy[k], h, f2_fma(wy[k], A, xy[k]));
+    m[k] = fmaf(f2_get(wy[k]).x, cm, m[k]);
+    A = f2_add(A, e);
+  }
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) k_p2g(Batch B) {
+  SCENE_CTA(B, MAP_P);
+  using Y = P2GLayout<D>;
+  constexpr int NN = Y::NN, PN = Y::PN, TN = Y::TN, NC = 1 << (2 * D);
+  constexpr unsigned ALL = 0xffffffffu;
+  extern __shared__ float4 dsm4[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float* area = (float*)dsm4 + warp * Y::WARP_FLOATS;
+  float4* sums = (float4*)area;               // [TASKS][NN]
+  float4* tiles = (float4*)(area + Y::AREA);  // [GROUPS][TN]
+  const int nitem = c.ctr[CTR_ITEMS];
+  const long long nw = (long long)nblk_ * Y::WARPS, wid = (long long)bid_ * Y::WARPS + warp;
+  const int i0 = (int)(wid * nitem / nw), i1 = (int)((wid + 1) * nitem / nw);
+  if (i0 >= i1) return;
+  const float radius = c.radius, r2 = 2.f * radius;
+  const float kw = (D == 2) ? 1.f / (4.f * r2 * r2) : 1.f / (8.f * r2 * r2 * r2);
+  const float pw = (D == 2) ? 0.25f : 0.125f;                            // 0.5**dim
+  const float rd = (D == 2) ? radius * radius : radius * radius * radius;  // radius**dim
+  const bool half = radius == 0.5f;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int t = lane; t < Y::GROUPS * TN; t += 32) tiles[t] = zero;
+  // step 2: this lane's task and plane
+  const int mytask = lane / Y::SPLIT, n0 = lane % Y::SPLIT;
+  // step 3: this lane's node and task group
+  const int grp = lane / NN, node = lane % NN;
+  const unsigned gmask = grp < Y::GROUPS ? ((1u << NN) - 1u) << (grp * NN) : 0u;
+  int toff = 0;  // the node's offset in the tile
+#pragma unroll
+  for (int d = 0, r = node, m = 1; d < D; ++d, r /= 3, m *= 6) toff += (r % 3) * m;
+  float4* tile = tiles + (grp < Y::GROUPS ? grp : 0) * TN + toff;
+  int bin = -1, excl = 0, nt0 = 0, off0 = 0, off1 = 0, c0 = 0, c1 = 0, tasks = 0, bstart = 0;
+  int4 it = c.items[i0];
+  for (int i = i0; i < i1; ++i) {
+    const int l = it.x & 15, lt = (it.x >> 4) & 15, first = (it.x >> 8) * Y::TASKS, blk = it.y;
+    if (it.z != bin) {
+      // the bin's cells: lane holds cells 2 lane, 2 lane + 1 (3D) or cell
+      // lane (2D): their particles, and the tasks of the cells before them
+      bin = it.z;
+      bstart = c.bin_start[bin];
+      const int* co = c.cell_off + (long long)bin * NC;
+      if (D == 3) {
+        const int2 o = *(const int2*)(co + 2 * lane);
+        off0 = o.x;
+        off1 = o.y;
+      } else {
+        off0 = off1 = lane < NC ? co[lane] : it.w;
+      }
+      int nx = __shfl_down_sync(ALL, off0, 1);
+      if (lane == 31) nx = it.w;
+      c0 = (D == 3 ? off1 : nx) - off0;
+      c1 = D == 3 ? nx - off1 : 0;
+      nt0 = (c0 + (1 << lt) - 1) >> lt;
+      const int nt = nt0 + ((c1 + (1 << lt) - 1) >> lt);
+      int inc = nt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(ALL, inc, o);
+        if (lane >= o) inc += y;
+      }
+      excl = inc - nt;
+      tasks = __shfl_sync(ALL, inc, 31);
+    }
+    int total = it.w;  // the bin's particles
+    if (i + 1 < i1) it = c.items[i + 1];
+    // lane t < TASKS holds task first + t: its cell, first particle and particles
+    const int k = first + lane;
+    int own = 0;  // the last lane whose cells start at or before task k
+#pragma unroll
+    for (int s = 16; s; s >>= 1)
+      if (__shfl_sync(ALL, excl, own + s) <= k) own += s;
+    int j = k - __shfl_sync(ALL, excl, own);
+    const int ont0 = __shfl_sync(ALL, nt0, own);
+    int off = __shfl_sync(ALL, off0, own), n = __shfl_sync(ALL, c0, own), cell = own;
+    if (D == 3) {
+      const int o1 = __shfl_sync(ALL, off1, own), m1 = __shfl_sync(ALL, c1, own);
+      cell = 2 * own;
+      if (j >= ont0) {
+        j -= ont0;
+        off = o1;
+        n = m1;
+        ++cell;
+      }
+    }
+    const int nv = min(Y::TASKS, tasks - first);  // tasks of this item
+    const int start = lane < nv ? off + (j << lt) : 0x7fffffff;
+    const int cnt = lane < nv ? min(1 << lt, n - (j << lt)) : 0;
+    const int s0 = __shfl_sync(ALL, start, 0), e0 = __shfl_sync(ALL, start + cnt, nv - 1);
+    // place in the tile of the cell's first node
+    const int place = D == 3 ? ((cell >> 4) * 6 + ((cell >> 2) & 3)) * 6 + (cell & 3) : (cell >> 2) * 6 + (cell & 3);
+    // the next item's particles follow this one's in the bin, or start the next
+    // bin; 3D asks for them ahead of the sums (2 to 3 percent; 2D items are over
+    // before it helps)
+    int ahead[2] = {-1, -1};
+    if (D == 3 && i + 1 < i1) {
+      int from = bstart + e0, left = total - e0;
+      if (it.z != bin) {
+        from = c.bin_start[it.z];
+        left = it.w;
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        if (32 * r + lane < left) ahead[r] = __ldg(&c.perm[from + 32 * r + lane]);
+    }
+    // -- 1. records -------------------------------------------------------------
+    {
+      const float inv = (float)(c.coarsest << l);
+      const float sc = 2.f * ((-c.dt * pw) / (rd * (1.f / inv)));
+      const int* perm = c.perm + bstart;
+#pragma unroll 1
+      for (int p0 = s0; p0 < e0; p0 += 32) {
+        const int q = p0 + lane;
+        int task = 0;  // the last task that starts at or before q
+#pragma unroll
+        for (int s = 8; s; s >>= 1)
+          if (__shfl_sync(ALL, start, task + s) <= q) task += s;
+        const int ts = __shfl_sync(ALL, start, task);
+        if (q < e0) p2g_record<D>(c, __ldg(&perm[q]), inv, sc, area + (q - ts) * Y::ROW + task * Y::REC);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (D == 3 && ahead[r] >= 0) {
+        const float4* src = c.P.s + prow<D>(ahead[r]);
+#pragma unroll
+        for (int k = 0; k < PWord<D>::NQ; ++k) asm volatile("prefetch.global.L2 [%0];" ::"l"(src + 32 * k));
+      }
+    __syncwarp();
+    // -- 2. sums of the lane's plane ------------------------------------------------
+    {
+      const int count = __shfl_sync(ALL, cnt, mytask);
+      const float* R = area + mytask * Y::REC;
+      f2 xy[PN], zm[D == 3 ? PN : 1];
+      float m[D == 2 ? PN : 1];
+#pragma unroll
+      for (int a = 0; a < PN; ++a) {
+        xy[a] = 0ull;
+        if (D == 3) zm[a % (D == 3 ? PN : 1)] = 0ull;
+        if (D == 2) m[a % (D == 2 ? PN : 1)] = 0.f;
+      }
+#pragma unroll 1
+      for (int p = 0; p < count; ++p, R += Y::ROW) {
+        if constexpr (D == 3)
+          p2g_plane(R, radius, half, n0, xy, zm);
+        else
+          p2g_row(R, radius, half, n0, xy, m);
+      }
+      __syncwarp();  // the records have been read: the sums take their place
+      if (mytask < nv)
+#pragma unroll
+        for (int a = 0; a < PN; ++a) {
+          const float2 u = f2_get(xy[a]);
+          float2 w;
+          if constexpr (D == 3)
+            w = f2_get(zm[a]);
+          else
+            w = make_float2(0.f, m[a]);
+          sums[mytask * NN + n0 * PN + a] = make_float4(u.x, u.y, w.x, w.y);
+        }
+    }
+    __syncwarp();
+    // -- 3. lane <-> node: the tasks of one cell, then the tile ---------------------
+    {
+      const int per = (nv + Y::GROUPS - 1) / Y::GROUPS;
+      const int j0 = grp * per;
+      float4 acc = zero;
+      int at = -1;  // place of the cell being summed
+      auto flush = [&]() {
+        float4 o = tile[at];
+        o.x += acc.x;
+        o.y += acc.y;
+        if (D == 3) o.z += acc.z;
+        o.w += acc.w;
+        tile[at] = o;
+        __syncwarp(gmask);  // the lanes of one tile stay together
+      };
+#pragma unroll 2
+      for (int e = 0; e < per; ++e) {
+        const int tj = j0 + e;
+        const int pj = __shfl_sync(ALL, place, tj & 31);
+        if (grp >= Y::GROUPS || tj >= nv) continue;
+        const float4 v = sums[tj * NN + node];
+        if (pj != at) {
+          if (at >= 0) flush();
+          at = pj;
+          acc = v;
+        } else {
+          acc.x += v.x;
+          acc.y += v.y;
+          if (D == 3) acc.z += v.z;
+          acc.w += v.w;
+        }
+      }
+      if (at >= 0) flush();
+    }
+    __syncwarp();
+    // the same block follows: keep summing into the tile
+    if (i + 1 < i1 && it.y == blk && (it.x & 15) == l) continue;
     const LevelDev& V = c.lev[l];
     int O[D];
-    chunk_origin<D>(V, wd.y, O);
-    float* tile = tiles + tb * 4 * Y::TN;
-    // -- 1. per-particle records -----------------------------------------------
-    const int i = threadIdx.x;
-    int cell = -1;
-    if (i < wd.w) {
-      const int p = __ldg(&c.perm[wd.z + i]);
-      const float inv = (float)(c.coarsest << l);
-      const float dx = 1.f / inv;
-      using PW = PWord<D>;
-      float4 st[PW::NQ];
-      const float4* src = c.P.s + prow<D>(p);
+    chunk_origin<D>(V, blk, O);
+    for (int t = lane; t < TN; t += 32) {
+      float4 val = tiles[t];
+      tiles[t] = zero;
 #pragma unroll
-      for (int k = 0; k < PW::NQ; ++k) st[k] = __ldg(src + 32 * k);
-      float xp[D], vp[D], F[D * D], Cm[D * D];
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        xp[d] = qword(st, PW::X + d);
-        vp[d] = qword(st, PW::V + d);
+      for (int g = 1; g < Y::GROUPS; ++g) {
+        const float4 o = tiles[g * TN + t];
+        tiles[g * TN + t] = zero;
+        val.x += o.x;
+        val.y += o.y;
+        val.w += o.w;
       }
-#pragma unroll
-      for (int k = 0; k < D * D; ++k) {
-        F[k] = qword(st, PW::F + k);
-        Cm[k] = qword(st, PW::C + k);
-      }
-      const float mp = qword(st, PW::M);
-      const float jp = qword(st, PW::JP);
-      float tc[D];
-      cell = 0;
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        const float xs = xp[d] * inv;
-        const int base = (int)(xs + 0.5f) - 1;
-        tc[d] = xs - (float)(base + 1);
-        cell = (cell << 2) | ((base - O[d]) & 3);
-      }
-      float mu = c.mu, la = c.la;
-      if (c.plast == 1) {
-        const float h = expf(c.xi * (1.f - jp));
-        mu *= h;
-        la *= h;
-      }
-      const float J = det<D>(F);
-      float tau[(D == 2) ? 3 : 6];
-      kirchhoff_sym<D>(F, 2.f * mu, la * J * (J - 1.f), tau);
-      const float sc = (-c.dt * pw) / (rd * dx);
-      float a[D];
-#pragma unroll
-      for (int r = 0; r < D; ++r) {
-        float cd = 0.f;
-#pragma unroll
-        for (int b = 0; b < D; ++b) cd += Cm[r * D + b] * (tc[b] + 1.f);
-        a[r] = mp * (vp[r] - cd);
-      }
-      // axis factors, scaled so that a node's weight is the product of its
-      // W's and the gradient's factors need no constant: axis 0 carries kw,
-      // every G carries kg / kw = 2
-      float W[D][3], G[D][3];
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        if (half)
-          axis_weights_half(tc[d], W[d], G[d]);
-        else
-          axis_weights(tc[d], c.radius, W[d], G[d]);
-        const float sw = d == 0 ? kw : 1.f;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          W[d][k] *= sw;
-          G[d][k] *= 2.f * sw;
-        }
-      }
-      float4* P4 = (float4*)(pd + i * Y::STRIDE);
-      const float cf = __int_as_float(cell);
-      if (D == 3) {
-        // row r = 3 n0 + n1: A = cw (a + B[:,0] n0 + B[:,1] n1) + S[:,0] cg0 + S[:,1] cg1
-        // with cw = W0[n0] W1[n1], cg0 = G0[n0] W1[n1], cg1 = W0[n0] G1[n1]
-        const float Bx0 = mp * Cm[0], By0 = mp * Cm[D], Bz0 = mp * Cm[(2 * D) % (D * D)];
-        const float Bx1 = mp * Cm[1], By1 = mp * Cm[D + 1], Bz1 = mp * Cm[(2 * D + 1) % (D * D)];
-        const float Sxx = sc * tau[0], Sxy = sc * tau[1], Syy = sc * tau[2];
-        const float Sxz = sc * tau[3 % (D == 3 ? 6 : 3)], Syz = sc * tau[4 % (D == 3 ? 6 : 3)];
-        const float Szz = sc * tau[5 % (D == 3 ? 6 : 3)];
-#pragma unroll
-        for (int r0 = 0; r0 < 3; ++r0) {
-#pragma unroll
-          for (int r1 = 0; r1 < 3; ++r1) {
-            const float cw = W[0][r0] * W[1][r1], cg0 = G[0][r0] * W[1][r1], cg1 = W[0][r0] * G[1][r1];
-            const float fn0 = (float)r0, fn1 = (float)r1;
-            const float ux = fmaf(Bx1, fn1, fmaf(Bx0, fn0, a[0]));
-            const float uy = fmaf(By1, fn1, fmaf(By0, fn0, a[1]));
-            const float uz = fmaf(Bz1, fn1, fmaf(Bz0, fn0, a[D - 1]));
-            P4[3 * r0 + r1] = make_float4(fmaf(cw, ux, fmaf(Sxx, cg0, Sxy * cg1)),
-                                          fmaf(cw, uy, fmaf(Sxy, cg0, Syy * cg1)),
-                                          fmaf(cw, uz, fmaf(Sxz, cg0, Syz * cg1)), cw);
-          }
-        }
-        P4[9] = make_float4(mp * Cm[2 % (D * D)], mp * Cm[(D + 2) % (D * D)], mp * Cm[D * D - 1], mp);
-        P4[10] = make_float4(Sxz, Syz, Szz, cf);
-        P4[11] = make_float4(W[D - 1][0], W[D - 1][1], W[D - 1][2], G[D - 1][0]);
-        *(float2*)(P4 + 12) = make_float2(G[D - 1][1], G[D - 1][2]);
-      } else {
-        // row r = n0: A = cw (a + B[:,0] n0) + S[:,0] cg0 with cw = W0[n0], cg0 = G0[n0]
-        const float Bx0 = mp * Cm[0], By0 = mp * Cm[D];
-        const float Sxx = sc * tau[0], Sxy = sc * tau[1], Syy = sc * tau[2];
-#pragma unroll
-        for (int r0 = 0; r0 < 3; ++r0) {
-          const float cw = W[0][r0], cg0 = G[0][r0], fn0 = (float)r0;
-          const float ux = fmaf(Bx0, fn0, a[0]), uy = fmaf(By0, fn0, a[1]);
-          P4[r0] = make_float4(fmaf(cw, ux, Sxx * cg0), fmaf(cw, uy, Sxy * cg0), cw, cf);
-        }
-        P4[3] = make_float4(mp * Cm[1], mp * Cm[D + 1 < D * D ? D + 1 : 0], Sxy, Syy);
-        P4[4] = make_float4(W[D - 1][0], W[D - 1][1], W[D - 1][2], mp);
-        P4[5] = make_float4(G[D - 1][0], G[D - 1][1], G[D - 1][2], 0.f);
-      }
-    }
-    __syncwarp();
-    // -- 2. this warp's particles in SLOTS ranges, lane <-> node row -------------
-    const int wbase = warp * 32;
-    const int nvalid = max(0, min(32, wd.w - wbase));
-    auto walk = [&](const int j0, const int j1) {
-      float2 axy[3];
-      float az[3], am[3];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        axy[k] = make_float2(0.f, 0.f);
-        az[k] = am[k] = 0.f;
-      }
-      int cur = -1;
-#pragma unroll 2
-      for (int j = j0; j < j1; ++j) {
-        const float* R = pd + (wbase + j) * Y::STRIDE;
-        const float4 rw = *(const float4*)(R + 4 * row);  // this row's A (and cw, 2D: and the cell)
-        const float4 sl = D == 3 ? *(const float4*)(R + 40) : make_float4(0.f, 0.f, 0.f, 0.f);  // SL, cell
-        const int cc = __float_as_int(D == 3 ? sl.w : rw.w);
-        if (cc != cur) {
-          // Cells ascend with the row axis fastest: the next cell one or two
-          // steps further along the same line shares the row's last nodes,
-          // so only the nodes it leaves behind go to the tile and the others
-          // move down the row.
-          const int dz = cc - cur;
-          if (cur >= 0 && (cc >> 2) == (cur >> 2) && dz > 0 && dz < 3) {
-            const int ti = p2g_row_tile<D>(cur, n0, n1);
-            p2g_node_flush<D>(tile, Y::TN, ti, axy[0], az[0], am[0]);
-            if (dz == 2) p2g_node_flush<D>(tile, Y::TN, ti + 1, axy[1], az[1], am[1]);
-            const float2 zz = make_float2(0.f, 0.f);
-            axy[0] = dz == 1 ? axy[1] : axy[2];
-            az[0] = dz == 1 ? az[1] : az[2];
-            am[0] = dz == 1 ? am[1] : am[2];
-            axy[1] = dz == 1 ? axy[2] : zz;
-            az[1] = dz == 1 ? az[2] : 0.f;
-            am[1] = dz == 1 ? am[2] : 0.f;
-            axy[2] = zz;
-            az[2] = am[2] = 0.f;
-          } else {
-            if (cur >= 0) p2g_row_flush<D>(tile, Y::TN, cur, n0, n1, axy, az, am);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-              axy[k] = make_float2(0.f, 0.f);
-              az[k] = am[k] = 0.f;
-            }
-          }
-          cur = cc;
-        }
-        // Node k of the row has weight cw wL[k] and gradient
-        // (cg_0 wL[k], .., cg_{d-2} wL[k], cw gL[k]); its momentum term is
-        //   w (a + B n) + S grad w = wL[k] (A + k Bk) + gL[k] s_L
-        // with A = cw (a + B n_row) + sum_{b<d-1} S[:, b] cg_b (the record's
-        // row part), Bk = cw B[:, d-1] and s_L = cw S[:, d-1]; the mass term
-        // is wL[k] cw m.
-        float wL[3], gL[3], cw, mp;
-        float2 Axy, bkxy, slxy;
-        if (D == 3) {
-          const float4 bm = *(const float4*)(R + 36);           // Bk_x Bk_y Bk_z m
-          const float4 wl = *(const float4*)(R + 44);           // W2[0..2] G2[0]
-          const float2 gh = *(const float2*)(R + 48);           // G2[1] G2[2]
-          wL[0] = wl.x, wL[1] = wl.y, wL[2] = wl.z;
-          gL[0] = wl.w, gL[1] = gh.x, gL[2] = gh.y;
-          cw = rw.w;
-          mp = bm.w;
-          Axy = make_float2(rw.x, rw.y);
-          bkxy = fmul2(dup2(cw), make_float2(bm.x, bm.y));
-          slxy = fmul2(dup2(cw), make_float2(sl.x, sl.y));
-          const float Az = rw.z, bkz = cw * bm.z, slz = cw * sl.z;
-          az[0] = fmaf(gL[0], slz, fmaf(wL[0], Az, az[0]));
-          az[1] = fmaf(gL[1], slz, fmaf(wL[1], Az + bkz, az[1]));
-          az[2] = fmaf(gL[2], slz, fmaf(wL[2], fmaf(2.f, bkz, Az), az[2]));
-        } else {
-          const float4 bs = *(const float4*)(R + 12);  // Bk_x Bk_y SL_x SL_y
-          const float4 wl = *(const float4*)(R + 16);  // W1[0..2] m
-          const float4 gl = *(const float4*)(R + 20);  // G1[0..2]
-          wL[0] = wl.x, wL[1] = wl.y, wL[2] = wl.z;
-          gL[0] = gl.x, gL[1] = gl.y, gL[2] = gl.z;
-          cw = rw.z;
-          mp = wl.w;
-          Axy = make_float2(rw.x, rw.y);
-          bkxy = fmul2(dup2(cw), make_float2(bs.x, bs.y));
-          slxy = fmul2(dup2(cw), make_float2(bs.z, bs.w));
-        }
-        const float2 A1xy = fadd2(Axy, bkxy), A2xy = ffma2(dup2(2.f), bkxy, Axy);
-        axy[0] = ffma2(dup2(gL[0]), slxy, ffma2(dup2(wL[0]), Axy, axy[0]));
-        axy[1] = ffma2(dup2(gL[1]), slxy, ffma2(dup2(wL[1]), A1xy, axy[1]));
-        axy[2] = ffma2(dup2(gL[2]), slxy, ffma2(dup2(wL[2]), A2xy, axy[2]));
-        const float cm = cw * mp;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) am[k] = fmaf(wL[k], cm, am[k]);
-      }
-      if (cur >= 0) p2g_row_flush<D>(tile, Y::TN, cur, n0, n1, axy, az, am);
-    };
-    if (D == 3) {
-      // 3D: SLOTS equal ranges of consecutive particles in one pass (11, 11,
-      // 10)
-      if (q < Y::SLOTS) walk((q * nvalid) / Y::SLOTS, ((q + 1) * nvalid) / Y::SLOTS);
-    } else {
-      // 2D: runs of one base cell (found with ballots, at most TMAX long; a
-      // cell holds about 4 particles), SLOTS runs at a time, one tile update
-      // per run (equal ranges of 3-4 particles would mostly straddle two
-      // cells: twice the tile updates)
-      const bool valid = lane < nvalid;
-      const int prev = __shfl_up_sync(0xffffffffu, cell, 1);
-      const unsigned runs = __ballot_sync(0xffffffffu, valid && (lane == 0 || cell != prev));
-      const int rs = valid ? 31 - __clz(runs & ((2u << lane) - 1u)) : 0;  // start of this lane's run
-      const bool tstart = valid && (lane - rs) % Y::TMAX == 0;
-      const unsigned tmask = __ballot_sync(0xffffffffu, tstart);
-      const int ntask = __popc(tmask);
-      int* ws = starts + warp * 33;  // task k starts at ws[k]; ws[ntask] = nvalid
-      if (tstart) ws[__popc(tmask & ((1u << lane) - 1u))] = lane;
-      if (lane == 0) ws[ntask] = nvalid;
-      __syncwarp();
-      for (int t0 = 0; t0 < ntask; t0 += Y::SLOTS) {
-        const int t = t0 + q;
-        if (q < Y::SLOTS && t < ntask) walk(ws[t], ws[t + 1]);
-      }
-    }
-    // the next work item's step 1 overwrites this warp's records and task
-    // starts, which lanes of this warp may still be reading above
-    __syncwarp();
-    if (!last) continue;  // the same block follows: keep summing into this tile
-    __syncthreads();
-    // -- 3. flush and clear ---------------------------------------------------
-    for (int t = threadIdx.x; t < Y::TN; t += blockDim.x) {
-      const float4 val = make_float4(tile[t], tile[Y::TN + t], D == 3 ? tile[2 * Y::TN + t] : 0.f, tile[3 * Y::TN + t]);
       if (val.x == 0.f && val.y == 0.f && val.z == 0.f && val.w == 0.f) continue;
-      int I[D];
-      int tt = t;
+      int I[D], tt = t;
 #pragma unroll
       for (int d = D - 1; d >= 0; --d) {
         I[d] = O[d] + tt % 6;
         tt /= 6;
       }
-      tile[t] = tile[Y::TN + t] = tile[3 * Y::TN + t] = 0.f;
-      if (D == 3) tile[2 * Y::TN + t] = 0.f;
       if (!in_store<D>(V, I)) {
         set_err(c, ERR_OOB);
         continue;
       }
-      atomicAdd(&V.node[elem_of<D>(V, I)], val);
+      atomicAdd(&V.node[elem_of<D>(V, I)], make_float4(val.x * kw, val.y * kw, val.z * kw, val.w * kw));
     }
-    tb ^= 1;
+    __syncwarp();
   }
 }
 
@@ -1435,7 +1505,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
   g2p_finish<D>(c, l, p, j, st, nv, G);
 }
 
-// 3D G2P (adaptive_gimp.py:289-321) over the P2G work items: a CTA takes a
+// 3D G2P (adaptive_gimp.py:289-321) over its work items (k_offsets): a CTA takes a
 // contiguous range of them (up to CH particles of one 4^3 block each); when
 // the block changes it stages the block's 6^3 node velocities in shared
 // memory (two tiles alternate, so one barrier per block suffices: a thread
@@ -1521,53 +1591,30 @@ __global__ void __launch_bounds__(256) k_project(Batch B) {
 }
 
 // ---------------------------------------------------------------------------
-template <int D, int CH>
+template <int D>
 static void set_p2g_smem() {
-  cudaFuncSetAttribute(k_p2g<D, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2GLayout<D, CH>::bytes());
+  cudaFuncSetAttribute(k_p2g<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P2GLayout<D>::bytes());
 }
 
-// CTAs of k_p2g<dim, chunk> that one SM holds at once (shared memory bound)
-int p2g_resident(int dim, int chunk) {
+// CTAs of k_p2g that one SM holds at once
+int p2g_resident(int dim) {
   int n = 0;
-  auto occ = [&](auto k, int ch, size_t smem) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, ch, smem); };
-  if (dim == 2) {
-    switch (chunk) {
-      case 64: occ(k_p2g<2, 64>, 64, P2GLayout<2, 64>::bytes()); break;
-      case 128: occ(k_p2g<2, 128>, 128, P2GLayout<2, 128>::bytes()); break;
-      case 512: occ(k_p2g<2, 512>, 512, P2GLayout<2, 512>::bytes()); break;
-      default: occ(k_p2g<2, 256>, 256, P2GLayout<2, 256>::bytes()); break;
-    }
-  } else {
-    switch (chunk) {
-      case 64: occ(k_p2g<3, 64>, 64, P2GLayout<3, 64>::bytes()); break;
-      case 128: occ(k_p2g<3, 128>, 128, P2GLayout<3, 128>::bytes()); break;
-      case 512: occ(k_p2g<3, 512>, 512, P2GLayout<3, 512>::bytes()); break;
-      default: occ(k_p2g<3, 256>, 256, P2GLayout<3, 256>::bytes()); break;
-    }
-  }
+  if (dim == 2)
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_p2g<2>, 32 * P2GLayout<2>::WARPS, P2GLayout<2>::bytes());
+  else
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_p2g<3>, 32 * P2GLayout<3>::WARPS, P2GLayout<3>::bytes());
   return n > 0 ? n : 1;
 }
 
 void prepare_transfer_kernels() {
-  set_p2g_smem<2, 64>();
-  set_p2g_smem<2, 128>();
-  set_p2g_smem<2, 256>();
-  set_p2g_smem<3, 64>();
-  set_p2g_smem<3, 128>();
-  set_p2g_smem<3, 256>();
-  set_p2g_smem<2, 512>();
-  set_p2g_smem<3, 512>();
+  set_p2g_smem<2>();
+  set_p2g_smem<3>();
 }
 
 template <int D>
 static void launch_p2g(const BatchLaunch& bl, cudaStream_t s, bool pdl) {
-  const int G = bl.nct[MAP_P];
-  switch (bl.chunk) {
-    case 64: launch_k(pdl, k_p2g<D, 64>, G, 64, P2GLayout<D, 64>::bytes(), s, bl.b); break;
-    case 128: launch_k(pdl, k_p2g<D, 128>, G, 128, P2GLayout<D, 128>::bytes(), s, bl.b); break;
-    case 512: launch_k(pdl, k_p2g<D, 512>, G, 512, P2GLayout<D, 512>::bytes(), s, bl.b); break;
-    default: launch_k(pdl, k_p2g<D, 256>, G, 256, P2GLayout<D, 256>::bytes(), s, bl.b); break;
-  }
+  using Y = P2GLayout<D>;
+  launch_k(pdl, k_p2g<D>, bl.nct[MAP_P], 32 * Y::WARPS, Y::bytes(), s, bl.b);
 }
 
 template <int D>

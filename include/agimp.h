@@ -91,7 +91,7 @@ typedef struct agimp_params {
 typedef struct agimp_stats {
   int32_t active_blocks[8]; /* 4^dim-cell blocks visited per level in the last substep */
   int32_t n_binned;         /* particles with fl_p >= 0 in the last substep */
-  int32_t n_chunks;         /* P2G/G2P work items in the last substep */
+  int32_t n_chunks;         /* G2P work items in the last substep */
   int64_t substeps;         /* substeps run since creation */
   int32_t n_surrogate;      /* particles whose return map went to the surrogate MLP (last substep) */
   int32_t n_fallback;       /* of those, predictions rejected for the exact return map */
@@ -333,7 +333,7 @@ agimp_status agimp_cell_lines(agimp_sim* s, float* vertices, int64_t capacity, i
  * launch sizes).  Results do not depend on it beyond the order of float
  * additions. */
 typedef struct agimp_tuning {
-  int32_t chunk;        /* particles per P2G work item (CTA size): 64, 128, 256 or 512 */
+  int32_t chunk;        /* particles per 3D G2P work item (CTA size): 64, 128, 256 or 512 */
   int32_t ctas_per_sm;  /* CTAs of the grid-stride kernels per multiprocessor, 1..32 */
   float ms_per_substep; /* the autotuner's measurement of this choice (else as set) */
 } agimp_tuning;
