@@ -3,12 +3,11 @@
 // autotuner.  A single simulator steps through this same path as a batch of
 // one.
 //
-// Launch layout.  Each launch kind (grid-stride kernels, the bin allocator)
-// gives every scene a consecutive range of CTAs:
+// Launch layout.  Each launch kind (grid-stride kernels, staged level
+// transfers, P2G) gives every scene a consecutive range of CTAs:
 //   grid-stride kernels (over particles, active blocks or work items):
 //     sms * ctas_per_sm CTAs shared in proportion to the scenes' particle
-//     counts (at least one each);
-//   bin allocator: a quarter of the scene's grid-stride CTAs (at least one).
+//     counts (at least one each).
 // The kernels find their scene by binary search over the range starts.
 #include <cstdlib>
 #include <algorithm>
@@ -173,10 +172,9 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
   // wait for one another), four for a batch (the scenes' shares are whole CTAs)
   const long long GP = (long long)b->sms * p2g_resident(b->dim) * (n == 1 ? 1 : 4);
   int* Gm = b->hofs.data() + MAP_G * (n + 1);
-  int* O = b->hofs.data() + MAP_O * (n + 1);
   int* T = b->hofs.data() + MAP_T * (n + 1);
   int* Pm = b->hofs.data() + MAP_P * (n + 1);
-  Gm[0] = O[0] = T[0] = Pm[0] = 0;
+  Gm[0] = T[0] = Pm[0] = 0;
   auto share = [&](long long tot, long long N) {
     return n == 1 ? (int)std::max<long long>(1, tot)
                   : (int)std::max<long long>(1, sumN ? (long long)std::llround((double)tot * N / sumN) : 1);
@@ -185,12 +183,10 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
     const long long N = b->sims[i]->c.N;
     const int cg = share(G, N);
     Gm[i + 1] = Gm[i] + cg;
-    O[i + 1] = O[i] + std::max(1, cg / 4);
     T[i + 1] = T[i] + 4 * cg;
     Pm[i + 1] = Pm[i] + share(GP, N);
   }
   b->nct[MAP_G] = Gm[n];
-  b->nct[MAP_O] = O[n];
   b->nct[MAP_T] = T[n];
   b->nct[MAP_P] = Pm[n];
   BCK(cudaMemcpyAsync(b->dofs, b->hofs.data(), sizeof(int) * b->hofs.size(), cudaMemcpyHostToDevice, use));

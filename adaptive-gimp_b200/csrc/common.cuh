@@ -57,9 +57,8 @@ enum {
   CTR_SURFB = 15,  // surrogate predictions rejected (exact return map used instead)
   // [16, 22): particle bounding box used by the refinement rule
   CTR_PROJ = 22,   // particles whose trial state needs the return map this substep
-  CTR_FULL = 23,   // non-empty bins this substep (listed in full_bins)
-  CTR_ITEMS = 24,  // P2G work items this substep
-  CTR_COUNT = 25
+  CTR_ITEMS = 23,  // P2G work items this substep
+  CTR_COUNT = 24
 };
 
 struct LevelDev {
@@ -270,13 +269,10 @@ struct Ctx {
   uint32_t* touch_flag;
   int32_t* touch_list;
   uint32_t* touch_occ;  // static mode, [finest blocks][1 (2D) or 5 (3D)]: base cells of the block's particles
-  int32_t* bin_count;   // [bins]: particles per bin
   int32_t* cell_count;  // [bins][4^d]: particles per (bin, base cell inside the bin's block)
-  int32_t* cell_off;    // [bins][4^d]: their offsets inside the bin (particles of a bin are cell-sorted)
-  int32_t* bin_start;
-  int32_t* full_bins;   // [bins]: the non-empty bins of this substep
+  int32_t* cell_off;    // [bins][4^d]: their first particle in bin order (a bin's particles are cell-sorted)
   int4* chunks;  // {level, block (stored linear id), start, count}
-  int4* items;   // P2G: {level | log2 T << 4 | item of the bin << 8, block (stored linear id), bin, particles of the bin}
+  int4* items;   // P2G: {level | log2 T << 4 | item of the bin << 8, block (stored linear id), bin, end of the bin's particles}
   int32_t* bin_of;      // per particle: bin * 4^d + base cell
   int32_t* rank_of;
   int32_t* perm;
@@ -429,6 +425,21 @@ __device__ __forceinline__ uint32_t nm_get(const Ctx& c, int l, const int* I) {
     if (P[d] < 0 || P[d] > c.sz) return 0u;
   }
   return c.nmask[elem_of<D>(c.lev[c.L - 1], P)];
+}
+
+// the node mask's word of node I of level l; null outside the finest lattice
+// [0, sz], where it is never read by a predicate
+template <int D>
+__device__ __forceinline__ uint32_t* nm_word(const Ctx& c, int l, const int* I) {
+  const int s = c.L - 1 - l;
+  int P[D];
+  bool in = true;
+#pragma unroll
+  for (int d = 0; d < D; ++d) {
+    P[d] = I[d] * (1 << s);
+    in = in && P[d] >= 0 && P[d] <= c.sz;
+  }
+  return in ? &c.nmask[elem_of<D>(c.lev[c.L - 1], P)] : nullptr;
 }
 
 template <int D>
@@ -1046,10 +1057,9 @@ __host__ __device__ __forceinline__ void axis_weights_half(float t, float* W, fl
 // consecutive ranges, one per scene; a CTA finds its scene by binary search
 // over the range starts and copies the scene's context into shared memory.
 enum { MAP_G = 0,  // grid-stride kernels over particles, active blocks or work items
-       MAP_O = 1,  // bin allocation (1024-thread CTAs)
-       MAP_T = 2,  // staged level transfers (one 4^d block per CTA at a time: 4x MAP_G's CTAs)
-       MAP_P = 3,  // P2G: one wave (batches: four) of the CTAs that fit the SMs at once
-       NMAP = 4 };
+       MAP_T = 1,  // staged level transfers (one 4^d block per CTA at a time: 4x MAP_G's CTAs)
+       MAP_P = 2,  // P2G: one wave (batches: four) of the CTAs that fit the SMs at once
+       NMAP = 3 };
 
 struct Batch {
   const Ctx* ctx;  // [n] scene contexts in device memory

@@ -7,7 +7,7 @@
 //   98-124  _mark_hier_ / _split_hier_-> k_mark_hier + k_resolve
 //   142-153 _activate_mask            -> k_resolve (same pass)
 //   155-187 ghost / T-junction        -> k_ghost_tj (all levels in one pass)
-//   189-216 level_mapping             -> k_bin + k_offsets + k_scatter
+//   189-216 level_mapping             -> k_bin + k_bins + k_scatter
 //
 // The reference runs its sparse sweeps level by level.  Here each pass covers
 // every level at once: the reads each pass depends on are not written in the
@@ -52,7 +52,6 @@ __global__ void k_clear(Batch B) {
     c.ctr[CTR_SURFB] = 0;
     if (c.sur) *c.sur_ctr = 0;  // a batch's shared slot counter (every scene clears it)
     c.ctr[CTR_PROJ] = 0;
-    c.ctr[CTR_FULL] = 0;
     c.ctr[CTR_ITEMS] = 0;
   }
   __shared__ BlockRanges br;
@@ -587,7 +586,7 @@ __global__ void k_level_masks(Batch B) {
 // ACTIVATED cell among the 2^d cells around the particle; bin = (fl_p, block
 // of base).  Particles without a level go to one extra bin after all block
 // bins, so that every particle gets a slot in the new order.  The rank inside
-// the bin comes from a warp-aggregated atomic.
+// the bin's cell comes from a warp-aggregated atomic.
 // lb: lb[l] = bins of the levels below l (block bins are numbered level by
 // level); lb[L] = all block bins, the index of the extra bin
 template <int D>
@@ -605,6 +604,7 @@ __device__ __forceinline__ void bin_one(const Ctx& c, int p, const int* lb) {
     int fl = -1;
     if (!esc) {
       // the finest level with an ACTIVATED cell: search from the finest down
+      // (two levels' words at a time take longer, 40 -> 44 us for 1.9M particles)
       for (int l = c.L - 1; l >= 0 && fl < 0; --l) {
         const float inv = (float)(c.coarsest << l);
         int base[D];
@@ -642,12 +642,7 @@ __device__ __forceinline__ void bin_one(const Ctx& c, int p, const int* lb) {
     if (fl < 0) bin = lb[c.L] << (2 * D);  // the extra bin
     c.P.fl[p] = fl;
   }
-  // bin sizes and the rank inside the (bin, cell): warp-aggregated atomics
-  {
-    const int b = bin >= 0 ? bin >> (2 * D) : -1;
-    const unsigned gb = __match_any_sync(0xffffffffu, b);
-    if (b >= 0 && lane == __ffs(gb) - 1) atomicAdd(&c.bin_count[b], __popc(gb));
-  }
+  // the rank inside the (bin, cell): warp-aggregated atomics
   const unsigned grp = __match_any_sync(0xffffffffu, bin);
   const int leader = __ffs(grp) - 1;
   const int rank = __popc(grp & ((1u << lane) - 1u));
@@ -677,150 +672,123 @@ __global__ void k_bin(Batch B) {
 }
 
 // ---------------------------------------------------------------------------
-// Bin storage: each CTA scans 1024 bins, reserves their particles and work
-// items with one atomic each, and writes the work-item descriptors.  Bins of
-// different CTAs land in any order; a bin's particles stay contiguous.
-__device__ __forceinline__ int2 block_incl_scan2(int a, int b, int2* warp_sums) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int ya = __shfl_up_sync(0xffffffffu, a, o);
-    const int yb = __shfl_up_sync(0xffffffffu, b, o);
-    if (lane >= o) {
-      a += ya;
-      b += yb;
-    }
-  }
-  if (lane == 31) warp_sums[w] = make_int2(a, b);
-  __syncthreads();
-  if (w == 0) {
-    const int nw = blockDim.x >> 5;
-    int2 s = lane < nw ? warp_sums[lane] : make_int2(0, 0);
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int ya = __shfl_up_sync(0xffffffffu, s.x, o);
-      const int yb = __shfl_up_sync(0xffffffffu, s.y, o);
-      if (lane >= o) {
-        s.x += ya;
-        s.y += yb;
-      }
-    }
-    if (lane < nw) warp_sums[lane] = s;
-  }
-  __syncthreads();
-  if (w > 0) {
-    const int2 pre = warp_sums[w - 1];
-    a += pre.x;
-    b += pre.y;
-  }
-  return make_int2(a, b);
-}
-
+// Bin storage: the first particle of every (bin, cell) (a bin's particles are
+// stored in cell order), the G2P work items (chunks) and the P2G work items (up
+// to P2G_TASKS tasks of up to 2^p2g_log_task particles of one cell each).  A
+// warp takes 4 (3D: its lanes hold two cells each) or 8 bins (2D: half-warps,
+// one cell each) at a time, which reserve their particles and items together,
+// with one atomic per counter (a counter that every bin bumps serialises at
+// L2).  Bins of different warps land in any order; a bin's particles stay
+// contiguous.  Cell counts are cleared for the next substep.  Bound by the
+// latency of two dependent L2 round trips, so the rounds' loads are issued
+// together.  Two kernels before (a scan over per-bin counts, which cost k_bin a
+// second atomic per particle group, then the cells' offsets): 20,000 2D
+// particles 9.5 -> 5.4 us, 256 2D scenes 33 -> 30 us, and k_bin with 1.9M 3D
+// particles 46 -> 40 us, with 15.5M 330 -> 300 us.
 template <int D>
-__global__ void __launch_bounds__(1024) k_offsets(Batch B) {
-  SCENE_CTA(B, MAP_O);
-  __shared__ int2 warp_sums[32];
-  __shared__ int2 s_base;
-  const int CH = c.chunk;
-  long long nblk = 0;
-  for (int q = 0; q < c.L; ++q) nblk += c.ctr[CTR_LEVEL + q];
-  const long long nb = nblk + 1;  // block bins + the extra bin of particles without a level
-  for (long long t0 = (long long)bid_ * blockDim.x; t0 < nb; t0 += (long long)nblk_ * blockDim.x) {
-    const long long b = t0 + threadIdx.x;
-    int cnt = 0;
-    if (b < nb) {
-      cnt = c.bin_count[b];
-      if (cnt) c.bin_count[b] = 0;
+__global__ void __launch_bounds__(256) k_bins(Batch B) {
+  SCENE_CTA(B, MAP_G);
+  constexpr int LANES = D == 3 ? 32 : 16;  // lanes of a bin
+  constexpr int GROUPS = 32 / LANES, ROUNDS = 4;
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, sub = lane & (LANES - 1), group = lane / LANES;
+  const int wid = bid_ * (blockDim.x >> 5) + (threadIdx.x >> 5), nw = nblk_ * (blockDim.x >> 5);
+  int nblocks = 0;
+  for (int q = 0; q < c.L; ++q) nblocks += c.ctr[CTR_LEVEL + q];
+  const int nbins = nblocks + 1, CH = c.chunk;  // and the bin of particles without a level
+  for (int b0 = wid * ROUNDS * GROUPS; b0 < nbins; b0 += nw * ROUNDS * GROUPS) {
+    int2 cells[ROUNDS];  // this lane's cells (2D: the first)
+    bool any = false;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      const int b = b0 + r * GROUPS + group;
+      cells[r] = make_int2(0, 0);
+      if (b < nbins) {
+        if (D == 3)
+          cells[r] = *(const int2*)(c.cell_count + ((long long)b << 6) + 2 * sub);
+        else
+          cells[r].x = c.cell_count[((long long)b << 4) + sub];
+      }
+      any = any || cells[r].x || cells[r].y;
     }
-    const int nch = (cnt + CH - 1) / CH;
-    const int2 inc = block_incl_scan2(cnt, nch, warp_sums);
-    if (threadIdx.x == blockDim.x - 1) {
-      s_base.x = inc.x ? atomicAdd(&c.ctr[CTR_BINCUR], inc.x) : 0;
-      s_base.y = inc.y ? atomicAdd(&c.ctr[CTR_CHUNKS], inc.y) : 0;
+    if (!__any_sync(ALL, any)) continue;
+    // per bin: particles before this lane's cells, all particles, tasks; the
+    // bins' shares before it in the warp's reservation
+    int before[ROUNDS], total[ROUNDS], tasks[ROUNDS], log_task[ROUNDS];
+    int np = 0, nc = 0, ni = 0;
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      const int mine = cells[r].x + cells[r].y;
+      int inc = mine, used = (cells[r].x > 0) + (cells[r].y > 0);
+#pragma unroll
+      for (int o = 1; o < LANES; o <<= 1) {
+        const int y = __shfl_up_sync(ALL, inc, o, LANES);
+        if (sub >= o) inc += y;
+        used += __shfl_xor_sync(ALL, used, o, LANES);
+      }
+      total[r] = __shfl_sync(ALL, inc, LANES - 1, LANES);
+      before[r] = inc - mine;
+      const int lt = p2g_log_task(total[r] / max(used, 1), c.N);
+      int t = ((cells[r].x + (1 << lt) - 1) >> lt) + ((cells[r].y + (1 << lt) - 1) >> lt);
+#pragma unroll
+      for (int o = LANES / 2; o; o >>= 1) t += __shfl_xor_sync(ALL, t, o, LANES);
+      log_task[r] = lt;
+      // particles without a level have no P2G
+      tasks[r] = b0 + r * GROUPS + group < nblocks ? t : 0;
+      np += total[r];
+      nc += (total[r] + CH - 1) / CH;
+      ni += (tasks[r] + P2G_TASKS - 1) / P2G_TASKS;
     }
-    __syncthreads();
-    if (cnt > 0) {
-      const int start = s_base.x + inc.x - cnt;
-      c.bin_start[b] = start;
-      c.full_bins[reserve_slot(&c.ctr[CTR_FULL])] = (int)b;
-      const int ch0 = s_base.y + inc.y - nch;
-      int l = -1, blk = 0;  // level -1 marks the extra bin
-      if (b < nblk) {
+    // reservation: lanes 0, 1, 2 hold particles, chunks, items of all groups
+    int p0 = 0, c0 = 0, i0 = 0;  // the first half-warp's, for the second
+    const int op = __shfl_xor_sync(ALL, np, 16), oc = __shfl_xor_sync(ALL, nc, 16), oi = __shfl_xor_sync(ALL, ni, 16);
+    if (GROUPS == 2 && group == 1) {
+      p0 = op;
+      c0 = oc;
+      i0 = oi;
+    }
+    int base = 0;
+    if (lane < 3) {
+      const int n = lane == 0 ? np + (GROUPS == 2 ? op : 0) : lane == 1 ? nc + (GROUPS == 2 ? oc : 0)
+                                                                        : ni + (GROUPS == 2 ? oi : 0);
+      if (n) base = atomicAdd(&c.ctr[lane == 0 ? CTR_BINCUR : lane == 1 ? CTR_CHUNKS : CTR_ITEMS], n);
+    }
+    p0 += __shfl_sync(ALL, base, 0);
+    c0 += __shfl_sync(ALL, base, 1);
+    i0 += __shfl_sync(ALL, base, 2);
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      const int b = b0 + r * GROUPS + group;
+      if (total[r] == 0) continue;
+      const int first = p0 + before[r];
+      const long long row = (long long)b << (2 * D);
+      if (D == 3) {
+        *(int2*)(c.cell_off + row + 2 * sub) = make_int2(first, first + cells[r].x);
+        if (cells[r].x | cells[r].y) *(int2*)(c.cell_count + row + 2 * sub) = make_int2(0, 0);
+      } else {
+        c.cell_off[row + sub] = first;
+        if (cells[r].x) c.cell_count[row + sub] = 0;
+      }
+      int l = -1, blk = 0;  // level -1 marks the bin of particles without a level
+      if (b < nblocks) {
         l = 0;
-        long long r = b;
-        while (l < c.L - 1 && r >= c.ctr[CTR_LEVEL + l]) {
-          r -= c.ctr[CTR_LEVEL + l];
+        int k = b;
+        while (l < c.L - 1 && k >= c.ctr[CTR_LEVEL + l]) {
+          k -= c.ctr[CTR_LEVEL + l];
           ++l;
         }
-        blk = c.lev[l].blist[r];
-      } else {
-        c.ctr[CTR_UNBIN] = cnt;
+        blk = c.lev[l].blist[k];
+      } else if (sub == 0) {
+        c.ctr[CTR_UNBIN] = total[r];
       }
-      for (int j = 0; j < nch; ++j) c.chunks[ch0 + j] = make_int4(l, blk, start + j * CH, min(CH, cnt - j * CH));
+      for (int k = sub; k * CH < total[r]; k += LANES)
+        c.chunks[c0 + k] = make_int4(l, blk, p0 + k * CH, min(CH, total[r] - k * CH));
+      for (int k = sub; k * P2G_TASKS < tasks[r]; k += LANES)
+        c.items[i0 + k] = make_int4(l | (log_task[r] << 4) | (k << 8), blk, b, p0 + total[r]);
+      p0 += total[r];
+      c0 += (total[r] + CH - 1) / CH;
+      i0 += (tasks[r] + P2G_TASKS - 1) / P2G_TASKS;
     }
-    __syncthreads();
-  }
-}
-
-// Offsets of the cells inside each bin (the bin's particles are stored in
-// cell order) and the bin's P2G work items (up to P2G_TASKS tasks of up to
-// 2^p2g_log_task particles of one cell each); one warp per bin, cell counts cleared for the
-// next substep.
-template <int D>
-__global__ void k_cell_offsets(Batch B) {
-  SCENE_CTA(B, MAP_G);
-  constexpr int NC = 1 << (2 * D), PER = (NC + 31) / 32;
-  const int lane = threadIdx.x & 31;
-  const int wid = bid_ * (blockDim.x >> 5) + (threadIdx.x >> 5), nw = nblk_ * (blockDim.x >> 5);
-  const int nfull = c.ctr[CTR_FULL];
-  int nblk = 0;
-  for (int q = 0; q < c.L; ++q) nblk += c.ctr[CTR_LEVEL + q];
-  for (int t = wid; t < nfull; t += nw) {
-    const int b = c.full_bins[t];
-    int* cc = c.cell_count + ((long long)b << (2 * D));
-    int n[PER], tot = 0, used = 0;
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int cell = lane * PER + k;
-      n[k] = cell < NC ? cc[cell] : 0;
-      tot += n[k];
-      used += n[k] > 0;
-    }
-    int inc = tot;  // inclusive scan of the lanes' totals
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += y;
-    }
-    int run = inc - tot;
-    int* co = c.cell_off + ((long long)b << (2 * D));
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-      const int cell = lane * PER + k;
-      if (cell < NC) {
-        co[cell] = run;
-        run += n[k];
-        if (n[k]) cc[cell] = 0;
-      }
-    }
-    if (b >= nblk) continue;  // the bin of particles without a level: no transfer
-    const int total = __shfl_sync(0xffffffffu, inc, 31);
-    const int lt = p2g_log_task(total / __reduce_add_sync(0xffffffffu, used), c.N);
-    int tasks = 0;
-#pragma unroll
-    for (int k = 0; k < PER; ++k) tasks += (n[k] + (1 << lt) - 1) >> lt;
-    tasks = __reduce_add_sync(0xffffffffu, tasks);
-    const int ni = (tasks + P2G_TASKS - 1) / P2G_TASKS;
-    int i0 = 0;
-    if (lane == 0) i0 = atomicAdd(&c.ctr[CTR_ITEMS], ni);
-    i0 = __shfl_sync(0xffffffffu, i0, 0);
-    int l = 0, r = b;
-    while (l < c.L - 1 && r >= c.ctr[CTR_LEVEL + l]) {
-      r -= c.ctr[CTR_LEVEL + l];
-      ++l;
-    }
-    const int blk = c.lev[l].blist[r];
-    for (int k = lane; k < ni; k += 32) c.items[i0 + k] = make_int4(l | (lt << 4) | (k << 8), blk, b, total);
   }
 }
 
@@ -828,8 +796,7 @@ template <int D>
 __global__ void k_scatter(Batch B) {
   SCENE_CTA(B, MAP_G);
   SCENE_LOOP(p, c.N) {
-    const int key = c.bin_of[p];
-    c.perm[c.bin_start[key >> (2 * D)] + c.cell_off[key] + c.rank_of[p]] = (int)p;
+    c.perm[c.cell_off[c.bin_of[p]] + c.rank_of[p]] = (int)p;
   }
 }
 
@@ -841,7 +808,7 @@ void launch_transfer(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev);
 template <int D>
 static void run_topology(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   const Batch& B = bl.b;
-  const int G = bl.nct[MAP_G], Go = bl.nct[MAP_O];
+  const int G = bl.nct[MAP_G];
   if (ev) cudaEventRecord(ev[0], s);
   const bool pdl = bl.pdl && !ev;
   // the first kernel follows whatever preceded the substep: a plain launch
@@ -864,8 +831,7 @@ static void run_topology(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev)
   if (ev) cudaEventRecord(ev[2], s);
   // after an event record or wait the next launch is a plain one
   launch_k(pdl && !bl.side, k_bin<D>, G, 256, 0, s, B);
-  launch_k(pdl, k_offsets<D>, Go, 1024, 0, s, B);
-  launch_k(pdl, k_cell_offsets<D>, G, 256, 0, s, B);
+  launch_k(pdl, k_bins<D>, G, 256, 0, s, B);
   launch_k(pdl, k_scatter<D>, G, 256, 0, s, B);
   if (ev) cudaEventRecord(ev[3], s);
 }
@@ -880,6 +846,8 @@ void launch_substep(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   }
 }
 
+// passes of a substep: a kernel each, but for the two of the bins' offsets
+// (particles per bin, cells inside it), which share k_bins
 int kernels_per_substep(const BatchLaunch& bl) {
   const int topo = 10 - (bl.any_dynamic ? 0 : 1) + (bl.dim == 3 && bl.maxL > 1 ? 1 : 0);
   return topo + 2 + (bl.maxL == 1 ? 1 : 0) + (bl.any_plastic ? 1 : 0) + 2 * (bl.maxL - 1);

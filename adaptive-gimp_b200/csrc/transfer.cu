@@ -41,7 +41,7 @@ __device__ __forceinline__ void chunk_origin(const LevelDev& V, long long blk, i
 
 // ---------------------------------------------------------------------------
 // P2G (adaptive_gimp.py:230-250).  Each warp works alone on a contiguous range
-// of work items (k_cell_offsets): an item is up to TASKS tasks of one 4^d block
+// of work items (k_bins): an item is up to TASKS tasks of one 4^d block
 // of one level, a task up to T particles of one base cell (bins store their
 // particles sorted by cell, so an item's particles are contiguous).
 //  1. Rounds of 32 particles, one per lane: the scaled Kirchhoff stress S
@@ -103,7 +103,7 @@ __device__ __forceinline__ void p2g_record(const Ctx& c, int p, float inv, float
   float4 q[W::NQ];
   const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
-  for (int k = 0; k < W::NQ; ++k) q[k] = __ldg(src + 32 * k);
+  for (int k = 0; k < W::NQ; ++k) q[k] = src[32 * k];
   float t[D], F[D * D];
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
 #pragma unroll
   for (int d = 0, r = node, m = 1; d < D; ++d, r /= 3, m *= 6) toff += (r % 3) * m;
   float4* tile = tiles + (grp < Y::GROUPS ? grp : 0) * TN + toff;
-  int bin = -1, excl = 0, nt0 = 0, off0 = 0, off1 = 0, c0 = 0, c1 = 0, tasks = 0, bstart = 0;
+  int bin = -1, excl = 0, nt0 = 0, off0 = 0, off1 = 0, c0 = 0, c1 = 0, tasks = 0;
   int4 it = c.items[i0];
   for (int i = i0; i < i1; ++i) {
     const int l = it.x & 15, lt = (it.x >> 4) & 15, first = (it.x >> 8) * Y::TASKS, blk = it.y;
@@ -286,7 +286,6 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
       // the bin's cells: lane holds cells 2 lane, 2 lane + 1 (3D) or cell
       // lane (2D): their particles, and the tasks of the cells before them
       bin = it.z;
-      bstart = c.bin_start[bin];
       const int* co = c.cell_off + (long long)bin * NC;
       if (D == 3) {
         const int2 o = *(const int2*)(co + 2 * lane);
@@ -310,7 +309,7 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
       excl = inc - nt;
       tasks = __shfl_sync(ALL, inc, 31);
     }
-    int total = it.w;  // the bin's particles
+    const int bend = it.w;  // the end of the bin's particles
     if (i + 1 < i1) it = c.items[i + 1];
     // lane t < TASKS holds task first + t: its cell, first particle and particles
     const int k = first + lane;
@@ -342,20 +341,15 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
     // before it helps)
     int ahead[2] = {-1, -1};
     if (D == 3 && i + 1 < i1) {
-      int from = bstart + e0, left = total - e0;
-      if (it.z != bin) {
-        from = c.bin_start[it.z];
-        left = it.w;
-      }
+      const int from = it.z != bin ? c.cell_off[(long long)it.z * NC] : e0, left = (it.z != bin ? it.w : bend) - from;
 #pragma unroll
       for (int r = 0; r < 2; ++r)
-        if (32 * r + lane < left) ahead[r] = __ldg(&c.perm[from + 32 * r + lane]);
+        if (32 * r + lane < left) ahead[r] = c.perm[from + 32 * r + lane];
     }
     // -- 1. records -------------------------------------------------------------
     {
       const float inv = (float)(c.coarsest << l);
       const float sc = 2.f * ((-c.dt * pw) / (rd * (1.f / inv)));
-      const int* perm = c.perm + bstart;
 #pragma unroll 1
       for (int p0 = s0; p0 < e0; p0 += 32) {
         const int q = p0 + lane;
@@ -364,7 +358,7 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
         for (int s = 8; s; s >>= 1)
           if (__shfl_sync(ALL, start, task + s) <= q) task += s;
         const int ts = __shfl_sync(ALL, start, task);
-        if (q < e0) p2g_record<D>(c, __ldg(&perm[q]), inv, sc, area + (q - ts) * Y::ROW + task * Y::REC);
+        if (q < e0) p2g_record<D>(c, c.perm[q], inv, sc, area + (q - ts) * Y::ROW + task * Y::REC);
       }
     }
 #pragma unroll
@@ -1214,8 +1208,8 @@ __device__ __forceinline__ void copy_particle(const Ctx& c, int p, int j) {
   const float4* src = c.P.s + prow<D>(p);
   float4* dst = c.Q.s + prow<D>(j);
 #pragma unroll
-  for (int k = 0; k < PWord<D>::NQ; ++k) __stwb(dst + 32 * k, __ldg(src + 32 * k));
-  __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
+  for (int k = 0; k < PWord<D>::NQ; ++k) __stwb(dst + 32 * k, src[32 * k]);
+  __stwb(&c.Q.id[j], c.P.id[p]);
   __stwb(&c.Q.fl[j], -1);
 }
 
@@ -1274,7 +1268,7 @@ __device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, co
   float4* dst = c.Q.s + prow<D>(j);
 #pragma unroll
   for (int k = 0; k < W::NQ; ++k) __stwb(dst + 32 * k, make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
-  __stwb(&c.Q.id[j], __ldg(&c.P.id[p]));
+  __stwb(&c.Q.id[j], c.P.id[p]);
   __stwb(&c.Q.fl[j], l);
   // trial states that may leave the elastic interval get the return map in
   // k_project (it needs an SVD, whose registers would halve G2P's occupancy);
@@ -1287,8 +1281,8 @@ __device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, co
 // through L1 (particles of a bin share a (4+2)^d node tile).
 template <int D>
 __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
-  const int p = __ldg(&c.perm[j]);
-  const int l = __ldg(&c.P.fl[p]);
+  const int p = c.perm[j];
+  const int l = c.P.fl[p];
   if (l < 0) {
     copy_particle<D>(c, p, j);
     return;
@@ -1297,7 +1291,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
   const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
   for (int k = 0; k < 4; ++k)
-    if (D == 3 || k != 2) st[k] = __ldg(src + 32 * k);
+    if (D == 3 || k != 2) st[k] = src[32 * k];
   float xp[D];
 #pragma unroll
   for (int d = 0; d < D; ++d) xp[d] = qword(st, d);
@@ -1361,7 +1355,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
         if (D == 3) I[1] = base[1] + n1;
         I[D - 1] = base[D - 1] + k;
         // base lies in [-1, size-1] for an in-domain particle: always in store
-        const float4 nd = __ldg(&V.node[elem_of<D>(V, I)]);
+        const float4 nd = V.node[elem_of<D>(V, I)];
         const float gv[3] = {nd.x, nd.y, nd.z};
 #pragma unroll
         for (int i = 0; i < D; ++i) {
@@ -1505,7 +1499,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
   g2p_finish<D>(c, l, p, j, st, nv, G);
 }
 
-// 3D G2P (adaptive_gimp.py:289-321) over its work items (k_offsets): a CTA takes a
+// 3D G2P (adaptive_gimp.py:289-321) over its work items (k_bins): a CTA takes a
 // contiguous range of them (up to CH particles of one 4^3 block each); when
 // the block changes it stages the block's 6^3 node velocities in shared
 // memory (two tiles alternate, so one barrier per block suffices: a thread
@@ -1527,7 +1521,7 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
     const int i = threadIdx.x, j = wd.z + i;
     const bool mine = i < wd.w;
     if (wd.x < 0) {  // uniform over the CTA
-      if (mine) copy_particle<D>(c, __ldg(&c.perm[j]), j);
+      if (mine) copy_particle<D>(c, c.perm[j], j);
       continue;
     }
     const int l = wd.x;
@@ -1539,10 +1533,10 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
     int p = 0;
     float4 st[4];
     if (mine) {
-      p = __ldg(&c.perm[j]);
+      p = c.perm[j];
       const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) st[k] = __ldg(src + 32 * k);
+      for (int k = 0; k < 4; ++k) st[k] = src[32 * k];
     }
     if (l != tl || wd.y != tk) {  // uniform over the CTA
       tb ^= 1;
@@ -1556,7 +1550,7 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
           r /= 6;
         }
         float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (in_store<D>(V, I)) nd = __ldg(&V.node[elem_of<D>(V, I)]);
+        if (in_store<D>(V, I)) nd = V.node[elem_of<D>(V, I)];
         txy[tb][t] = make_float2(nd.x, nd.y);
         if (D == 3) tz[tb][t] = nd.z;
       }

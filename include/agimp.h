@@ -196,7 +196,8 @@ agimp_status agimp_get_node_mask(agimp_sim* s, int32_t* out, int32_t memory, voi
 agimp_status agimp_errors(agimp_sim* s, uint32_t* bits, int32_t clear);
 agimp_status agimp_get_stats(agimp_sim* s, agimp_stats* out);
 
-/* Number of kernels one substep launches (for launch accounting). */
+/* Number of passes of one substep (for launch accounting): a kernel each, but
+ * for the two passes over the bins' offsets, which are one launch. */
 int32_t agimp_kernels_per_substep(const agimp_sim* s);
 
 /* One substep with direct launches and CUDA events between its phases;
