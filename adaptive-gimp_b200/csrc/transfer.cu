@@ -470,10 +470,6 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
   }
 }
 
-// grid_op (adaptive_gimp.py:277-287) of node I of level l, stored at idx: an
-// activated node's momentum becomes its velocity (gravity, walls, colliders);
-// with inv_norm the other nodes with mass are divided by it.  I lies in
-// [0, size]^d.
 // Node mask of node I of level l stored at idx: 3D scenes read the level's
 // own copy (k_level_masks), which the staged transfers copy by whole blocks;
 // 2D scenes, whose transfers gather node by node, read the node mask itself.
@@ -483,14 +479,16 @@ __device__ __forceinline__ uint32_t level_mask(const Ctx& c, int l, const int* I
   return nm_get<D>(c, l, I);
 }
 
+// grid_op (adaptive_gimp.py:277-287) of node I of level l with mask nm and value
+// nd: an activated node's momentum becomes its velocity (gravity, walls,
+// colliders); with inv_norm the other nodes with mass are divided by it.  I lies
+// in [0, size]^d.
 template <int D>
-__device__ __forceinline__ void gridop_node(const Ctx& c, int l, const int* I, long long idx) {
-  const LevelDev& V = c.lev[l];
-  const float4 nd = V.node[idx];
-  if (!(nd.w > 0.f)) return;
-  if (!is_activated(level_mask<D>(c, l, I, idx))) {
-    if (c.inv_norm) V.node[idx] = make_float4(nd.x / nd.w, nd.y / nd.w, D == 3 ? nd.z / nd.w : nd.z, nd.w);
-    return;
+__device__ __forceinline__ float4 gridop_value(const Ctx& c, int l, const int* I, uint32_t nm, const float4 nd) {
+  if (!(nd.w > 0.f)) return nd;
+  if (!is_activated(nm)) {
+    if (c.inv_norm) return make_float4(nd.x / nd.w, nd.y / nd.w, D == 3 ? nd.z / nd.w : nd.z, nd.w);
+    return nd;
   }
   float vv[3] = {nd.x, nd.y, nd.z};
   const int s = c.L - 1 - l;
@@ -522,7 +520,14 @@ __device__ __forceinline__ void gridop_node(const Ctx& c, int l, const int* I, l
         for (int d = 0; d < D; ++d) vv[d] = 0.f;
     }
   }
-  V.node[idx] = make_float4(vv[0], vv[1], vv[2], nd.w);
+  return make_float4(vv[0], vv[1], vv[2], nd.w);
+}
+
+template <int D>
+__device__ __forceinline__ void gridop_node(const Ctx& c, int l, const int* I, long long idx) {
+  float4& node = c.lev[l].node[idx];
+  const uint32_t nm = level_mask<D>(c, l, I, idx);
+  node = gridop_value<D>(c, l, I, nm, node);
 }
 
 // ---------------------------------------------------------------------------
@@ -710,9 +715,13 @@ __global__ void __launch_bounds__(Stage<D>::PER) k_restrict(Batch B, int l) {
 // ---------------------------------------------------------------------------
 // The same two transfers as direct gathers through L1 (one thread per
 // destination node): used for 2D scenes, whose 16-node blocks are too small
-// for a staging round trip per block to pay.
+// for a staging round trip per block to pay.  Bound by the latency of L2
+// reads: a node's masks are loaded together, then the nodes they select
+// (before, each weight's mask and then its node: 20,000 particles restriction
+// 6.7 -> 4.4 us, prolongation 5.3 -> 4.0; 256 scenes 28 -> 26 and 31, as
+// before).  Three CTAs an SM: with two the batch takes 31 us (restriction).
 template <int D>
-__global__ void k_restrict_gather(Batch B, int l) {
+__global__ void __launch_bounds__(256, 3) k_restrict_gather(Batch B, int l) {
   SCENE_CTA(B, MAP_G);
   const bool restrict_l = l < c.L;
   if (!restrict_l && l != 1) return;
@@ -730,43 +739,65 @@ __global__ void k_restrict_gather(Batch B, int l) {
     for (int d = 0; d < D; ++d) inr = inr && K[d] >= 0 && K[d] <= l0sz;
     if (!inr) continue;
     const long long cidx = (blk << (2 * D)) | loc;
-    if (restrict_l && is_valid(level_mask<D>(c, l - 1, K, cidx))) {
+    const uint32_t cm = level_mask<D>(c, l - 1, K, cidx);
+    float4 o = Vc.node[cidx];
+    bool any = false;
+    if (restrict_l && is_valid(cm)) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      bool any = false;
+      // nine sources at a time (all in 2D, a plane in 3D): their masks are read
+      // together, then the nodes that count (two memory latencies)
 #pragma unroll
-      for (int a = 0; a < ((D == 2) ? 9 : 27); ++a) {
-        int I[D], nrm = 0, t = a;
-        bool ok = true;
+      for (int a0 = 0; a0 < ((D == 2) ? 9 : 27); a0 += 9) {
+        unsigned fidx[9], use = 0;
+        uint32_t nm[9];
+        auto weight = [&](int a, int* I) {  // source a's node and weight
+          int nrm = 0;
 #pragma unroll
-        for (int d = D - 1; d >= 0; --d) {
-          const int dI = t % 3 - 1;
-          t /= 3;
-          I[d] = 2 * K[d] - dI;
-          nrm += dI != 0;
-          ok = ok && I[d] >= 0 && I[d] <= lsz;
+          for (int d = D - 1; d >= 0; --d) {
+            const int dI = a % 3 - 1;
+            a /= 3;
+            I[d] = 2 * K[d] - dI;
+            nrm += dI != 0;
+          }
+          return (nrm == 0) ? 1.f : (nrm == 1) ? 0.5f : (nrm == 2) ? 0.25f : 0.125f;
+        };
+#pragma unroll
+        for (int a = 0; a < 9; ++a) {
+          int I[D];
+          weight(a0 + a, I);
+          bool ok = true;
+#pragma unroll
+          for (int d = 0; d < D; ++d) ok = ok && I[d] >= 0 && I[d] <= lsz;
+          fidx[a] = (unsigned)elem_of<D>(Vf, I);
+          nm[a] = ok ? level_mask<D>(c, l, I, fidx[a]) : 0u;
         }
-        if (!ok) continue;
-        const long long fidx = elem_of<D>(Vf, I);
-        const uint32_t nm = level_mask<D>(c, l, I, fidx);
-        if (!((is_activated(nm) && nrm == 0) || is_tj(nm) || is_ghost(nm))) continue;
-        const float w = (nrm == 0) ? 1.f : (nrm == 1) ? 0.5f : (nrm == 2) ? 0.25f : 0.125f;
-        const float4 f = Vf.node[fidx];
-        acc.x += f.x * w;
-        acc.y += f.y * w;
-        acc.z += f.z * w;
-        acc.w += f.w * w;
-        any = true;
+        float4 f[9];
+#pragma unroll
+        for (int a = 0; a < 9; ++a) {
+          int I[D];
+          if ((is_activated(nm[a]) && weight(a0 + a, I) == 1.f) || is_tj(nm[a]) || is_ghost(nm[a])) {
+            f[a] = Vf.node[fidx[a]];
+            use |= 1u << a;
+          }
+        }
+        any = any || use;
+#pragma unroll
+        for (int a = 0; a < 9; ++a) {
+          if (!(use >> a & 1u)) continue;
+          int I[D];
+          const float w = weight(a0 + a, I);
+          acc.x += f[a].x * w;
+          acc.y += f[a].y * w;
+          if (D == 3) acc.z += f[a].z * w;
+          acc.w += f[a].w * w;
+        }
       }
-      if (any) {
-        float4 o = Vc.node[cidx];
-        o.x += acc.x;
-        o.y += acc.y;
-        o.z += acc.z;
-        o.w += acc.w;
-        Vc.node[cidx] = o;
-      }
+      if (any) o = make_float4(o.x + acc.x, o.y + acc.y, o.z + acc.z, o.w + acc.w);
     }
-    if (l == 1) gridop_node<D>(c, 0, K, cidx);
+    if (l == 1)
+      Vc.node[cidx] = gridop_value<D>(c, 0, K, cm, o);
+    else if (any)
+      Vc.node[cidx] = o;
   }
 }
 
@@ -791,54 +822,51 @@ __global__ void k_prolong_gather(Batch B, int l) {
     }
     if (!inr) continue;
     const long long fidx = (blk << (2 * D)) | loc;
-    gridop_node<D>(c, l, J, fidx);
+    // the node and its mask are read together (even nodes: with the mask of the
+    // coarse node they take), then the masks of the coarse nodes around a T or
+    // ghost node, then the coarse nodes
+    const float4 nd = Vf.node[fidx];
     const uint32_t nm = level_mask<D>(c, l, J, fidx);
     const bool tg = is_tj(nm) || is_ghost(nm);
-    if (!tg && !even) continue;
-    float acc[3] = {0.f, 0.f, 0.f};
-    if (tg) {
-      int nodd = 0;
+    // node J lies between the coarse nodes J / 2 (and + 1 on its odd axes)
+    unsigned cidx[1 << D];
+    uint32_t cm[1 << D];
+    int nodd = 0;
 #pragma unroll
-      for (int d = 0; d < D; ++d) nodd += J[d] & 1;
-      const float w = (nodd == 0) ? 1.f : (nodd == 1) ? 0.5f : (nodd == 2) ? 0.25f : 0.125f;
+    for (int d = 0; d < D; ++d) nodd += J[d] & 1;
 #pragma unroll
-      for (int a = 0; a < (1 << D); ++a) {
-        int K[D];
-        bool use = true;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          const int bit = (a >> d) & 1;
-          if (J[d] & 1)
-            K[d] = (J[d] - 1) / 2 + bit;
-          else {
-            K[d] = J[d] / 2;
-            use = use && bit == 0;
-          }
-        }
-        if (!use) continue;
-        const long long cidx = elem_of<D>(Vc, K);
-        if (!is_valid(level_mask<D>(c, l - 1, K, cidx))) continue;
-        const float4 cv = Vc.node[cidx];
-        acc[0] += cv.x * w;
-        acc[1] += cv.y * w;
-        acc[2] += cv.z * w;
-      }
-    } else if (is_activated(nm)) {
+    for (int a = 0; a < (1 << D); ++a) {
       int K[D];
+      bool use = true;
 #pragma unroll
-      for (int d = 0; d < D; ++d) K[d] = J[d] / 2;
-      const long long cidx = elem_of<D>(Vc, K);
-      if (is_valid(level_mask<D>(c, l - 1, K, cidx))) {
-        const float4 cv = Vc.node[cidx];
-        acc[0] = cv.x;
-        acc[1] = cv.y;
-        acc[2] = cv.z;
+      for (int d = 0; d < D; ++d) {
+        const int bit = (a >> d) & 1;
+        K[d] = (J[d] >> 1) + bit;
+        use = use && (bit == 0 || (J[d] & 1));
       }
+      cidx[a] = (unsigned)elem_of<D>(Vc, K);
+      cm[a] = use && (even || tg) ? level_mask<D>(c, l - 1, K, cidx[a]) : 0u;
     }
-    float4 o = Vf.node[fidx];
-    o.x = acc[0];
-    o.y = acc[1];
-    o.z = acc[2];
+    float4 o = gridop_value<D>(c, l, J, nm, nd);
+    if (tg || even) {
+      const bool take = tg || is_activated(nm);  // (an even node's only source is a = 0)
+      const float w = (nodd == 0) ? 1.f : (nodd == 1) ? 0.5f : (nodd == 2) ? 0.25f : 0.125f;
+      float4 cv[1 << D];
+#pragma unroll
+      for (int a = 0; a < (1 << D); ++a)
+        if (take && is_valid(cm[a])) cv[a] = Vc.node[cidx[a]];
+      float acc[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int a = 0; a < (1 << D); ++a)
+        if (take && is_valid(cm[a])) {
+          acc[0] += cv[a].x * w;
+          acc[1] += cv[a].y * w;
+          if (D == 3) acc[2] += cv[a].z * w;
+        }
+      o.x = acc[0];
+      o.y = acc[1];
+      o.z = acc[2];
+    }
     Vf.node[fidx] = o;
   }
 }
