@@ -1012,6 +1012,101 @@ __host__ __device__ __forceinline__ bool gram_within(const float* S, float detF,
          S[5] + r2 <= hi2;
 }
 
+// Snow return map of a 3D F near a rotation (det F > 0, |F^T F - I|_F < 0.4):
+// clamps its singular values to [lo, hi] and updates Jp.  With E = F^T F - I =
+// V diag(e) V^T, sigma = sqrt(1 + e), the clamped F is F (I + K), K = V
+// diag(clamp(sigma) / sigma - 1) V^T, so neither U nor a rebuild from all of
+// U, sigma, V is needed, and errors of V count only times K's few percent:
+// Jacobi on E (Golub & Van Loan, Matrix Computations, 4th ed., Alg. 8.5.3) can
+// stop at off-diagonals of 3e-8 and use the hardware's reciprocal root, since
+// E's entries, unlike F^T F's, carry no rounding of the order of eps.  An F
+// inside the interval keeps its bits.  Returns false (nothing changed)
+// elsewhere; the caller then takes the SVD.
+__host__ __device__ __forceinline__ float rsqrt_fast(float x) {
+#ifdef __CUDA_ARCH__
+  return rsqrtf(x);
+#else
+  return 1.f / sqrtf(x);
+#endif
+}
+__host__ __device__ __forceinline__ float divide_fast(float a, float b) {
+#ifdef __CUDA_ARCH__
+  return __fdividef(a, b);
+#else
+  return a / b;
+#endif
+}
+// one rotation in the plane (p, q) of the symmetric matrix with diagonal
+// entries app, aqq, off-diagonal apq and the third axis' entries arp, arq
+__host__ __device__ __forceinline__ void jacobi_plane(float& app, float& aqq, float& apq, float& arp, float& arq,
+                                                      float* V, int p, int q) {
+  const float d = aqq - app, h2 = fmaf(d, d, 4.f * apq * apq);
+  const float h = h2 * rsqrt_fast(fmaxf(h2, 1e-36f));
+  const float t = divide_fast(copysignf(2.f, d) * apq, fabsf(d) + h + 1e-20f);
+  const float cs = rsqrt_fast(fmaf(t, t, 1.f)), sn = t * cs;
+  app = fmaf(-t, apq, app);
+  aqq = fmaf(t, apq, aqq);
+  apq = 0.f;
+  const float x = arp, y = arq;
+  arp = fmaf(cs, x, -sn * y);
+  arq = fmaf(sn, x, cs * y);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float a = V[3 * k + p], b = V[3 * k + q];
+    V[3 * k + p] = fmaf(cs, a, -sn * b);
+    V[3 * k + q] = fmaf(sn, a, cs * b);
+  }
+}
+__host__ __device__ __forceinline__ bool snow_clamp_near(float* F, float& jp, float lo, float hi) {
+  float e[6];  // E: xx, yy, zz, xy, xz, yz
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    e[i] = fmaf(F[6 + i], F[6 + i], fmaf(F[3 + i], F[3 + i], fmaf(F[i], F[i], -1.f)));
+    const int a = i == 2 ? 1 : 0, b = i == 0 ? 1 : 2;
+    e[3 + i] = fmaf(F[6 + a], F[6 + b], fmaf(F[3 + a], F[3 + b], F[a] * F[b]));
+  }
+  const float fro2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2] + 2.f * (e[3] * e[3] + e[4] * e[4] + e[5] * e[5]);
+  if (!(fro2 < 0.16f && det<3>(F) > 0.f)) return false;
+  float V[9] = {1.f, 0.f, 0.f, 0.f, 1.f, 0.f, 0.f, 0.f, 1.f};
+#pragma unroll 1
+  for (int sweep = 0; sweep < 6; ++sweep) {
+    if (fmaf(e[3], e[3], fmaf(e[4], e[4], e[5] * e[5])) <= 1e-15f) break;
+    jacobi_plane(e[0], e[1], e[3], e[4], e[5], V, 0, 1);
+    jacobi_plane(e[0], e[2], e[4], e[3], e[5], V, 0, 2);
+    jacobi_plane(e[1], e[2], e[5], e[3], e[4], V, 1, 2);
+  }
+  float k[3], Jo = 1.f, Jn = 1.f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const float sg = sqrtf(1.f + e[i]), cl = fminf(fmaxf(sg, lo), hi);
+    Jo *= sg;
+    Jn *= cl;
+    k[i] = divide_fast(cl - sg, sg);
+  }
+  if (k[0] == 0.f && k[1] == 0.f && k[2] == 0.f) return true;
+  jp = jp * Jo / Jn;
+  float K[6];  // as E
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int a = i == 2 ? 1 : 0, b = i == 0 ? 1 : 2;
+    K[i] = 0.f;
+    K[3 + i] = 0.f;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      K[i] = fmaf(k[m] * V[3 * i + m], V[3 * i + m], K[i]);
+      K[3 + i] = fmaf(k[m] * V[3 * a + m], V[3 * b + m], K[3 + i]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    const float x = F[3 * r], y = F[3 * r + 1], z = F[3 * r + 2];
+    F[3 * r] = x + fmaf(z, K[4], fmaf(y, K[3], x * K[0]));
+    F[3 * r + 1] = y + fmaf(z, K[5], fmaf(y, K[1], x * K[3]));
+    F[3 * r + 2] = z + fmaf(z, K[2], fmaf(y, K[5], x * K[4]));
+  }
+  return true;
+}
+
 // GIMP weights factorised per axis.  get_weight_stencil (adaptive_gimp.py:
 // 218-228) sums get_linear_weight (utils.py:18-42) over the 2^d cells dI and
 // 2^d corners cell_ that meet at node n = dI + cell_; the summand is a product

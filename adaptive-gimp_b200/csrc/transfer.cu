@@ -1149,7 +1149,9 @@ __device__ __forceinline__ bool sur_handoff(const Ctx& c, const float* U, const 
 // Snow return map of G2P's trial state F (in place): states whose singular
 // values are provably inside the clamp interval are unchanged; the others get
 // an SVD, are recorded when the recorder samples this particle, and are
-// projected exactly or handed to the surrogate.
+// projected exactly or handed to the surrogate.  (In 3D, G2P itself
+// projects the states near a rotation when neither recorder nor surrogate
+// wants their SVD.)
 template <int D>
 __device__ __forceinline__ void snow_return_map(const Ctx& c, float* F, float& jp, int j) {
   if (singular_values_within<D>(F, 1.f - c.theta_c, 1.f + c.theta_s)) return;
@@ -1286,23 +1288,40 @@ __device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, co
     w[W::V + d] = nv[d];
   }
 #pragma unroll
-  for (int k = 0; k < D * D; ++k) {
-    w[W::F + k] = Fn[k];
-    w[W::C + k] = G[k];
-  }
+  for (int k = 0; k < D * D; ++k) w[W::C + k] = G[k];
   w[W::M] = qword(st, W::M);
   w[W::G] = qword(st, W::G);
-  w[W::JP] = c.plast == 1 ? qword(st, W::JP) : 1.f;
   float4* dst = c.Q.s + prow<D>(j);
+  auto row = [&](int k) { __stwb(dst + 32 * k, make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3])); };
+  // the rows without F, Jp first: the return map needs the registers
 #pragma unroll
-  for (int k = 0; k < W::NQ; ++k) __stwb(dst + 32 * k, make_float4(w[4 * k], w[4 * k + 1], w[4 * k + 2], w[4 * k + 3]));
+  for (int k = 0; k < W::NQ; ++k)
+    if (D == 3 && (k == 0 || k > 3)) row(k);
   __stwb(&c.Q.id[j], c.P.id[p]);
   __stwb(&c.Q.fl[j], l);
-  // trial states that may leave the elastic interval get the return map in
-  // k_project (it needs an SVD, whose registers would halve G2P's occupancy);
-  // det F' = det(I + s G) det F
-  if (c.plast == 1 && !gram_within<D>(Sg, det<D>(A) * det<D>(F), 1.f - c.theta_c, 1.f + c.theta_s))
-    c.proj[reserve_slot(&c.ctr[CTR_PROJ])] = j;
+  // Trial states that may leave the elastic interval.  In 3D the ones near a
+  // rotation are projected here: it takes some 150 operations in the registers
+  // at hand.  Through the list and k_project it took another trip through
+  // memory and, with the SVD, 1000 operations (1.9M particles: G2P 97 + SVD 94
+  // us; G2P 98 + this projection in k_project 46; G2P with it 117).  The rest
+  // is listed for k_project, whose SVD would halve G2P's occupancy.
+  float jp = 1.f;
+  if (c.plast == 1) {
+    jp = qword(st, W::JP);
+    const float lo = 1.f - c.theta_c, hi = 1.f + c.theta_s;
+    // det F' = det(I + s G) det F
+    if (!gram_within<D>(Sg, det<D>(A) * det<D>(F), lo, hi)) {
+      bool done = false;
+      if constexpr (D == 3) done = !c.rec_X && !c.sur && snow_clamp_near(Fn, jp, lo, hi);
+      if (!done) c.proj[reserve_slot(&c.ctr[CTR_PROJ])] = j;
+    }
+  }
+  w[W::JP] = jp;
+#pragma unroll
+  for (int k = 0; k < D * D; ++k) w[W::F + k] = Fn[k];
+#pragma unroll
+  for (int k = 0; k < W::NQ; ++k)
+    if (!(D == 3 && (k == 0 || k > 3))) row(k);
 }
 
 // One particle, slot j of this substep's bin order; the 3^d nodes come
@@ -1588,8 +1607,10 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
   }
 }
 
-// Snow return map (extension) of the particles G2P listed: the trial state
-// written to Q is projected in place (or handed to the surrogate).
+// Snow return map (extension) of the particles G2P listed (2D: all that may
+// leave the elastic interval; 3D: those far from a rotation, or all when a
+// recorder or surrogate wants their SVD): the trial state written to Q is
+// projected in place (or handed to the surrogate).
 template <int D>
 __global__ void __launch_bounds__(256) k_project(Batch B) {
   SCENE_CTA(B, MAP_G);
