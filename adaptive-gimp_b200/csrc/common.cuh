@@ -27,7 +27,7 @@
 namespace agimp {
 
 constexpr int MAXL = 8;
-constexpr int CHUNK = 256;      // default G2P work item (particles of one bin) = 3D G2P CTA size
+constexpr int CHUNK = 128;      // default G2P work item (particles of one bin) = 3D G2P CTA size
 constexpr int MAX_CHUNK = 512;  // largest work item the tuning may choose
 constexpr int MIN_CHUNK = 64;   // smallest work item (sizes the work-item buffer)
 constexpr int HALO = 4;
@@ -1078,13 +1078,19 @@ __host__ __device__ __forceinline__ bool snow_clamp_near(float* F, float& jp, fl
   float k[3], Jo = 1.f, Jn = 1.f;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const float sg = sqrtf(1.f + e[i]), cl = fminf(fmaxf(sg, lo), hi);
+    // the root by one Newton step on y rsqrt(y) (sqrtf is a call here)
+    const float y = 1.f + e[i], r = rsqrt_fast(y), s0 = y * r;
+    const float sg = fmaf(0.5f * r, fmaf(-s0, s0, y), s0), cl = fminf(fmaxf(sg, lo), hi);
     Jo *= sg;
     Jn *= cl;
     k[i] = divide_fast(cl - sg, sg);
   }
   if (k[0] == 0.f && k[1] == 0.f && k[2] == 0.f) return true;
-  jp = jp * Jo / Jn;
+  {
+    // jp Jo / Jn, the quotient corrected by its remainder
+    const float a = jp * Jo, r = divide_fast(1.f, Jn), q = a * r;
+    jp = fmaf(r, fmaf(-q, Jn, a), q);
+  }
   float K[6];  // as E
 #pragma unroll
   for (int i = 0; i < 3; ++i) {

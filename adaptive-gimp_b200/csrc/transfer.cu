@@ -1243,18 +1243,38 @@ __device__ __forceinline__ void copy_particle(const Ctx& c, int p, int j) {
   __stwb(&c.Q.fl[j], -1);
 }
 
+// Factors of G2P that depend only on the scene and the level, computed once a
+// CTA (they hold four divisions, 5 % of G2P's time: 256 2D scenes 154 -> 141
+// us): s of F' = (I + s G) F per level, and the scale of the weights (kw) and
+// of their gradients (kg).
+struct G2PScale {
+  float s[MAXL], kw, kg;
+};
+template <int D>
+__device__ __forceinline__ void g2p_scale(const Ctx& c, G2PScale& sc) {
+  if ((int)threadIdx.x < c.L) {
+    const float pw = (D == 2) ? 0.25f : 0.125f;
+    const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;
+    const float dx = 1.f / (float)(c.coarsest << (int)threadIdx.x);
+    sc.s[threadIdx.x] = (c.dt * pw) / (rd * dx);
+  }
+  if (threadIdx.x == 32) {
+    const float r2 = 2.f * c.radius;
+    sc.kw = (D == 2) ? 1.f / (4.f * r2 * r2) : 1.f / (8.f * r2 * r2 * r2);
+    sc.kg = (D == 2) ? 1.f / (2.f * r2 * r2) : 1.f / (4.f * r2 * r2 * r2);
+  }
+  __syncthreads();
+}
+
 // The end of G2P for particle p (slot j of this substep's bin order, level l):
 // the new state from its position, node velocity nv and velocity gradient G
 // (F' = (I + s G) F, whose Gram matrix decides whether the snow return map
 // may change it).  st holds the rows of p before V (x, g, F, m, Jp).
 template <int D>
-__device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, const float4* st, const float* nv,
-                                           const float* G) {
+__device__ __forceinline__ void g2p_finish(const Ctx& c, const G2PScale& sc, int l, int p, int j, const float4* st,
+                                           const float* nv, const float* G) {
   using W = PWord<D>;
-  const float pw = (D == 2) ? 0.25f : 0.125f;
-  const float rd = (D == 2) ? c.radius * c.radius : c.radius * c.radius * c.radius;
-  const float dx = 1.f / (float)(c.coarsest << l);
-  const float s = (c.dt * pw) / (rd * dx);
+  const float s = sc.s[l];
   float F[D * D], A[D * D], Fn[D * D], Sg[(D == 2) ? 3 : 6];
 #pragma unroll
   for (int k = 0; k < D * D; ++k) F[k] = qword(st, W::F + k);
@@ -1303,7 +1323,7 @@ __device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, co
   // rotation are projected here: it takes some 150 operations in the registers
   // at hand.  Through the list and k_project it took another trip through
   // memory and, with the SVD, 1000 operations (1.9M particles: G2P 97 + SVD 94
-  // us; G2P 98 + this projection in k_project 46; G2P with it 117).  The rest
+  // us; G2P 98 + this projection in k_project 46; G2P with it 117, now 103).  The rest
   // is listed for k_project, whose SVD would halve G2P's occupancy.
   float jp = 1.f;
   if (c.plast == 1) {
@@ -1327,7 +1347,7 @@ __device__ __forceinline__ void g2p_finish(const Ctx& c, int l, int p, int j, co
 // One particle, slot j of this substep's bin order; the 3^d nodes come
 // through L1 (particles of a bin share a (4+2)^d node tile).
 template <int D>
-__device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
+__device__ __forceinline__ void g2p_one(const Ctx& c, const G2PScale& sc, int j) {
   const int p = c.perm[j];
   const int l = c.P.fl[p];
   if (l < 0) {
@@ -1376,9 +1396,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
       g = k == 0 ? Gk[0] : (k == 1 ? Gk[1] : Gk[2]);
     }
   };
-  const float r2 = 2.f * c.radius;
-  const float kw = (D == 2) ? 1.f / (4.f * r2 * r2) : 1.f / (8.f * r2 * r2 * r2);
-  const float kg = (D == 2) ? 1.f / (2.f * r2 * r2) : 1.f / (4.f * r2 * r2 * r2);
+  const float kw = sc.kw, kg = sc.kg;
   float nv[D], G[D * D];
 #pragma unroll
   for (int i = 0; i < D; ++i) nv[i] = 0.f;
@@ -1434,7 +1452,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
       }
     }
   }
-  g2p_finish<D>(c, l, p, j, st, nv, G);
+  g2p_finish<D>(c, sc, l, p, j, st, nv, G);
 }
 
 // 2D G2P: one thread per particle slot, grid-stride (a 2D block holds about
@@ -1442,7 +1460,9 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, int j) {
 template <int D>
 __global__ void __launch_bounds__(256, 4) k_g2p_gather(Batch B) {
   SCENE_CTA(B, MAP_G);
-  SCENE_LOOP(j, c.N) g2p_one<D>(c, (int)j);
+  __shared__ G2PScale sc;
+  g2p_scale<D>(c, sc);
+  SCENE_LOOP(j, c.N) g2p_one<D>(c, sc, (int)j);
 }
 
 // The new state of particle p (slot j of this substep's bin order) whose
@@ -1450,8 +1470,8 @@ __global__ void __launch_bounds__(256, 4) k_g2p_gather(Batch B) {
 // node velocities: txy[t] = (v_x, v_y), tz[t] = v_z of tile node t (the
 // (4+2)^d nodes O..O+5, last axis fastest).
 template <int D>
-__device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, const float4* st, const int* O,
-                                           const float2* txy, const float* tz) {
+__device__ __forceinline__ void g2p_staged(const Ctx& c, const G2PScale& sc, int l, int p, int j, const float4* st,
+                                           const int* O, const float2* txy, const float* tz) {
   const float inv = (float)(c.coarsest << l);
   float tc[D];
   int t0 = 0;
@@ -1487,9 +1507,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
       g = k == 0 ? Gk[0] : (k == 1 ? Gk[1] : Gk[2]);
     }
   };
-  const float r2 = 2.f * c.radius;
-  const float kw = (D == 2) ? 1.f / (4.f * r2 * r2) : 1.f / (8.f * r2 * r2 * r2);
-  const float kg = (D == 2) ? 1.f / (2.f * r2 * r2) : 1.f / (4.f * r2 * r2 * r2);
+  const float kw = sc.kw, kg = sc.kg;
   float nv[D], G[D * D];
 #pragma unroll
   for (int i = 0; i < D; ++i) nv[i] = 0.f;
@@ -1497,7 +1515,9 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
   for (int i = 0; i < D * D; ++i) G[i] = 0.f;
   // Rows along the last axis: a row's nodes are summed with the last axis's
   // weight (S) and gradient (T) first; the other axes' factors are applied
-  // once per row.
+  // once per row.  (Summing planes before the first axis as well saves a third
+  // of the multiply-adds, but its partial sums do not fit the 64 registers:
+  // 114 against 111 us for 1.9M particles, 34.6 against 30.7 for 300,000.)
 #pragma unroll
   for (int n0 = 0; n0 < 3; ++n0) {
     float w0, g0;
@@ -1543,7 +1563,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
       }
     }
   }
-  g2p_finish<D>(c, l, p, j, st, nv, G);
+  g2p_finish<D>(c, sc, l, p, j, st, nv, G);
 }
 
 // 3D G2P (adaptive_gimp.py:289-321) over its work items (k_bins): a CTA takes a
@@ -1556,19 +1576,38 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, int l, int p, int j, co
 template <int D, int CH>
 __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
   SCENE_CTA(B, MAP_G);
-  constexpr int TN = (D == 2) ? 36 : 216;
+  constexpr int TN = 216;
   __shared__ float2 txy[2][TN];
-  __shared__ float tz[2][(D == 3) ? TN : 1];
+  __shared__ float tz[2][TN];
+  __shared__ G2PScale sc;
+  g2p_scale<D>(c, sc);
+  __shared__ int4 item[32];
   const int nch = c.ctr[CTR_CHUNKS];
-  const int per = (nch + nblk_ - 1) / nblk_;
-  const int c0 = bid_ * per, c1 = min(nch, c0 + per);
-  int tb = 1, tl = -1, tk = -1;
+  const int q = nch / nblk_, extra = nch - q * nblk_;
+  const int c0 = bid_ * q + min(bid_, extra), c1 = c0 + q + (bid_ < extra);
+  const int i = threadIdx.x;
+  // The items of this CTA come 32 at a time through shared memory and a
+  // particle's source slot is read one item ahead, so an item starts with the
+  // reads of its particles' rows (300,000 static particles 27.4 -> 25.3 us).
+  // Items of 128 particles, not 256, halve the lanes idle in a block's last
+  // item (30.7 -> 27.4; 1.9M particles 111 -> 107); 64 load a tile for too few
+  // (33, 138).
+  auto source = [&](const int4& w) { return i < w.w ? c.perm[w.z + i] : 0; };
+  int tb = 1, tl = -1, tk = -1, next = 0;
   for (int ch = c0; ch < c1; ++ch) {
-    const int4 wd = c.chunks[ch];
-    const int i = threadIdx.x, j = wd.z + i;
+    const int k0 = (ch - c0) & 31;
+    if (k0 == 0) {
+      __syncthreads();
+      if (i < 32 && ch + i < c1) item[i] = c.chunks[ch + i];
+      __syncthreads();
+      next = source(item[0]);
+    }
+    const int4 wd = item[k0];
+    const int p = next, j = wd.z + i;
     const bool mine = i < wd.w;
     if (wd.x < 0) {  // uniform over the CTA
-      if (mine) copy_particle<D>(c, c.perm[j], j);
+      if (mine) copy_particle<D>(c, p, j);
+      if (k0 < 31 && ch + 1 < c1) next = source(item[k0 + 1]);
       continue;
     }
     const int l = wd.x;
@@ -1577,14 +1616,13 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
     chunk_origin<D>(V, wd.y, O);
     // the particle's rows before V are requested before the tile load, so both
     // latencies overlap
-    int p = 0;
     float4 st[4];
     if (mine) {
-      p = c.perm[j];
       const float4* src = c.P.s + prow<D>(p);
 #pragma unroll
       for (int k = 0; k < 4; ++k) st[k] = src[32 * k];
     }
+    if (k0 < 31 && ch + 1 < c1) next = source(item[k0 + 1]);
     if (l != tl || wd.y != tk) {  // uniform over the CTA
       tb ^= 1;
       tl = l;
@@ -1599,11 +1637,11 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
         float4 nd = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in_store<D>(V, I)) nd = V.node[elem_of<D>(V, I)];
         txy[tb][t] = make_float2(nd.x, nd.y);
-        if (D == 3) tz[tb][t] = nd.z;
+        tz[tb][t] = nd.z;
       }
       __syncthreads();
     }
-    if (mine) g2p_staged<D>(c, l, p, j, st, O, txy[tb], tz[tb]);
+    if (mine) g2p_staged<D>(c, sc, l, p, j, st, O, txy[tb], tz[tb]);
   }
 }
 
