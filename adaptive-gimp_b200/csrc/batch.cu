@@ -161,6 +161,20 @@ void batch_free(agimp_batch* b) {
   b->ev_in = b->ev_out = nullptr;
 }
 
+// MAP_W's CTAs as a multiple of MAP_G's, by the particles of all scenes.  With
+// one wave of resident CTAs the slowest share of the blocks or particles (a
+// CTA's blocks at level borders, a batch's scene with many of them) decides
+// when the kernel ends; with more, shorter ones the SMs fill up evenly, but
+// each wave costs some 1.5 us of prologues.  Times in us of ghost marks / bins
+// / G2P: 1.9M 3D particles, one wave 32 / 40 / 107, two 28 / 36 / 103, four 36
+// for the bins, 102 for G2P and 5 lost in the other kernels; 256 2D scenes, 5M:
+// one 45 / 60 / 141, four 38 / 52 / 133, eight 58 for the bins and 142 for G2P;
+// 15.5M 3D: one 114 / 297 / 784, four 247 for the bins and 736 for G2P, eight 94
+// / 242 / 717; the small scenes lose 2 to 3 us a kernel from the second wave on.
+static int launch_waves(long long particles) {
+  return particles < 1000000 ? 1 : particles < 4000000 ? 2 : particles < 10000000 ? 4 : 8;
+}
+
 // CTA ranges of every launch kind (host copy in b->hofs, uploaded on `use`).
 static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
   const int n = (int)b->sims.size();
@@ -174,7 +188,9 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
   int* Gm = b->hofs.data() + MAP_G * (n + 1);
   int* T = b->hofs.data() + MAP_T * (n + 1);
   int* Pm = b->hofs.data() + MAP_P * (n + 1);
-  Gm[0] = T[0] = Pm[0] = 0;
+  int* Wm = b->hofs.data() + MAP_W * (n + 1);
+  const int waves = launch_waves(sumN);
+  Gm[0] = T[0] = Pm[0] = Wm[0] = 0;
   auto share = [&](long long tot, long long N) {
     return n == 1 ? (int)std::max<long long>(1, tot)
                   : (int)std::max<long long>(1, sumN ? (long long)std::llround((double)tot * N / sumN) : 1);
@@ -184,11 +200,13 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
     const int cg = share(G, N);
     Gm[i + 1] = Gm[i] + cg;
     T[i + 1] = T[i] + 4 * cg;
+    Wm[i + 1] = Wm[i] + waves * cg;
     Pm[i + 1] = Pm[i] + share(GP, N);
   }
   b->nct[MAP_G] = Gm[n];
   b->nct[MAP_T] = T[n];
   b->nct[MAP_P] = Pm[n];
+  b->nct[MAP_W] = Wm[n];
   BCK(cudaMemcpyAsync(b->dofs, b->hofs.data(), sizeof(int) * b->hofs.size(), cudaMemcpyHostToDevice, use));
   b->maps_valid = true;
   return AGIMP_OK;

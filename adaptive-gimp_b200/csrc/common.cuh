@@ -1160,7 +1160,8 @@ __host__ __device__ __forceinline__ void axis_weights_half(float t, float* W, fl
 enum { MAP_G = 0,  // grid-stride kernels over particles, active blocks or work items
        MAP_T = 1,  // staged level transfers (one 4^d block per CTA at a time: 4x MAP_G's CTAs)
        MAP_P = 2,  // P2G: one wave (batches: four) of the CTAs that fit the SMs at once
-       NMAP = 3 };
+       MAP_W = 3,  // MAP_G's CTAs, several times over in large scenes (launch_waves): kernels whose elements differ in cost
+       NMAP = 4 };
 
 struct Batch {
   const Ctx* ctx;  // [n] scene contexts in device memory

@@ -42,7 +42,7 @@ __device__ __forceinline__ uint32_t cell_get(const Ctx& c, int l, const int* I) 
 // per-substep counters.
 template <int D>
 __global__ void k_clear(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   if (bid_ == 0 && threadIdx.x == 0) {
     c.ctr[CTR_TOUCH] = 0;
     c.ctr[CTR_BINCUR] = 0;
@@ -239,7 +239,7 @@ __device__ __forceinline__ void touch_one(const Ctx& c, int p) {
 
 template <int D>
 __global__ void k_touch_activate(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   // the active-block counts were read by k_clear; k_dilate rebuilds them
   if (bid_ == 0 && threadIdx.x < MAXL) c.ctr[CTR_LEVEL + threadIdx.x] = 0;
   SCENE_PARTICLES(p0) touch_one<D>(c, p0 + (int)threadIdx.x);
@@ -442,7 +442,7 @@ __global__ void k_mark_hier(Batch B) {
 // set until the next substep clears the block; readback masks it out.
 template <int D>
 __global__ void k_resolve(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   // k_dilate has read the touched blocks' reach: clear the flags for the next
   // substep (they are read again only by k_touch_activate)
   SCENE_LOOP(t, c.ctr[CTR_TOUCH]) {
@@ -519,7 +519,7 @@ __global__ void k_resolve(Batch B) {
 // _mark_ghost_and_T_junction for every level (adaptive_gimp.py:155-187).
 template <int D>
 __global__ void k_ghost_tj(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   __shared__ BlockRanges br;
   load_block_ranges(c, br);
   const long long tot = total_elems_r(br, 0, c.L, D);
@@ -629,7 +629,7 @@ __global__ void k_ghost_tj(Batch B) {
 // Runs after ghost / T-junction marking, the last writer of the node mask.
 template <int D>
 __global__ void k_level_masks(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   __shared__ BlockRanges br;
   load_block_ranges(c, br);
   const long long tot = total_elems_r(br, 0, c.L - 1, D);
@@ -723,7 +723,7 @@ __device__ __forceinline__ void bin_one(const Ctx& c, int p, const int* lb) {
 
 template <int D>
 __global__ void k_bin(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   __shared__ int lb[MAXL + 1];
   if (threadIdx.x == 0) {
     int t = 0;
@@ -874,29 +874,29 @@ void launch_transfer(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev);
 template <int D>
 static void run_topology(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   const Batch& B = bl.b;
-  const int G = bl.nct[MAP_G];
+  const int G = bl.nct[MAP_G], W = bl.nct[MAP_W];
   if (ev) cudaEventRecord(ev[0], s);
   const bool pdl = bl.pdl && !ev;
   // the first kernel follows whatever preceded the substep: a plain launch
-  launch_k(false, k_clear<D>, G, 256, 0, s, B);
-  launch_k(pdl, k_touch_activate<D>, G, 256, 0, s, B);
+  launch_k(false, k_clear<D>, W, 256, 0, s, B);
+  launch_k(pdl, k_touch_activate<D>, W, 256, 0, s, B);
   launch_k(pdl, k_dilate<D>, G, 256, 0, s, B);
   if (ev) cudaEventRecord(ev[1], s);
   if (bl.any_dynamic) launch_k(pdl, k_mark_hier<D>, G, 256, 0, s, B);
-  launch_k(pdl, k_resolve<D>, G, 256, 0, s, B);
+  launch_k(pdl, k_resolve<D>, W, 256, 0, s, B);
   if (bl.side) {
     cudaEventRecord(bl.fork, s);
     cudaStreamWaitEvent(bl.side, bl.fork, 0);
-    k_ghost_tj<D><<<G, 256, 0, bl.side>>>(B);
-    if (D == 3 && bl.maxL > 1) launch_k(true, k_level_masks<D>, G, 256, 0, bl.side, B);
+    launch_k(false, k_ghost_tj<D>, W, 256, 0, bl.side, B);
+    if (D == 3 && bl.maxL > 1) launch_k(true, k_level_masks<D>, W, 256, 0, bl.side, B);
     cudaEventRecord(bl.join, bl.side);
   } else {
-    launch_k(pdl, k_ghost_tj<D>, G, 256, 0, s, B);
-    if (D == 3 && bl.maxL > 1) launch_k(pdl, k_level_masks<D>, G, 256, 0, s, B);
+    launch_k(pdl, k_ghost_tj<D>, W, 256, 0, s, B);
+    if (D == 3 && bl.maxL > 1) launch_k(pdl, k_level_masks<D>, W, 256, 0, s, B);
   }
   if (ev) cudaEventRecord(ev[2], s);
   // after an event record or wait the next launch is a plain one
-  launch_k(pdl && !bl.side, k_bin<D>, G, 256, 0, s, B);
+  launch_k(pdl && !bl.side, k_bin<D>, W, 256, 0, s, B);
   launch_k(pdl, k_bins<D>, G, 256, 0, s, B);
   launch_k(pdl, k_scatter<D>, G, 256, 0, s, B);
   if (ev) cudaEventRecord(ev[3], s);

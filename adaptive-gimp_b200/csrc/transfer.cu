@@ -1459,7 +1459,7 @@ __device__ __forceinline__ void g2p_one(const Ctx& c, const G2PScale& sc, int j)
 // one work item, too little to pay for staging its nodes).
 template <int D>
 __global__ void __launch_bounds__(256, 4) k_g2p_gather(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   __shared__ G2PScale sc;
   g2p_scale<D>(c, sc);
   SCENE_LOOP(j, c.N) g2p_one<D>(c, sc, (int)j);
@@ -1575,7 +1575,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, const G2PScale& sc, int
 // Particles without a level (the extra bin) are copied unchanged.
 template <int D, int CH>
 __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
-  SCENE_CTA(B, MAP_G);
+  SCENE_CTA(B, MAP_W);
   constexpr int TN = 216;
   __shared__ float2 txy[2][TN];
   __shared__ float tz[2][TN];
@@ -1700,15 +1700,15 @@ static void launch_p2g(const BatchLaunch& bl, cudaStream_t s, bool pdl) {
 
 template <int D>
 static void launch_g2p(const BatchLaunch& bl, cudaStream_t s, bool pdl) {
-  const int G = bl.nct[MAP_G];
+  const int W = bl.nct[MAP_W];
   if constexpr (D == 2) {
-    launch_k(pdl, k_g2p_gather<D>, G, 256, 0, s, bl.b);
+    launch_k(pdl, k_g2p_gather<D>, W, 256, 0, s, bl.b);
   } else {
     switch (bl.chunk) {
-      case 64: launch_k(pdl, k_g2p<D, 64>, G, 64, 0, s, bl.b); break;
-      case 128: launch_k(pdl, k_g2p<D, 128>, G, 128, 0, s, bl.b); break;
-      case 512: launch_k(pdl, k_g2p<D, 512>, G, 512, 0, s, bl.b); break;
-      default: launch_k(pdl, k_g2p<D, 256>, G, 256, 0, s, bl.b); break;
+      case 64: launch_k(pdl, k_g2p<D, 64>, W, 64, 0, s, bl.b); break;
+      case 128: launch_k(pdl, k_g2p<D, 128>, W, 128, 0, s, bl.b); break;
+      case 512: launch_k(pdl, k_g2p<D, 512>, W, 512, 0, s, bl.b); break;
+      default: launch_k(pdl, k_g2p<D, 256>, W, 256, 0, s, bl.b); break;
     }
   }
 }
