@@ -33,8 +33,25 @@ Ctx& sim_ctx(agimp_sim* s) {
   return s->c;
 }
 
+// Grid-stride CTAs per SM before any tuning, by the particles of all scenes.  A
+// kernel of a small scene ends with its slowest chain of dependent reads, and
+// launching CTAs with nothing to do delays it by about 1 us per 1184; a larger
+// scene needs the warps.  Whole passes in us at 8 / 6 / 4 / 2 per SM: 21,000
+// particles (static 2D) 556 / 537 / 515 / 500, 27,000 (dynamic 2D) 740 / 731 /
+// 706 / 706, 81,000 (3D sphere) 594 / 554 / 549 / 563, 108,000 (dynamic 2D) 837
+// / 829 / 813 / 878, 195,000 (static 3D) 445 / 436 / 452 / 524, 316,000 (3D
+// sphere) 815 / 796 / 824 / 956, 358,000 (static 3D) 578 / 580 / 623 / 744.
+static int default_ctas(long long particles) {
+  return particles <= 32768 ? 2 : particles <= 131072 ? 4 : particles <= 327680 ? 6 : 8;
+}
+
 agimp_status batch_init(agimp_batch* b) {
   const int n = (int)b->sims.size();
+  {
+    long long sumN = 0;
+    for (agimp_sim* s : b->sims) sumN += s->c.N;
+    b->tune.ctas_per_sm = default_ctas(sumN);
+  }
   {
     const char* e = std::getenv("AGIMP_PDL");
     b->pdl = !(e && e[0] == '0');
@@ -182,7 +199,9 @@ static agimp_status build_maps(agimp_batch* b, cudaStream_t use) {
   for (agimp_sim* s : b->sims) sumN += s->c.N;
   const long long G = (long long)b->sms * b->tune.ctas_per_sm;
   // P2G: one wave of resident CTAs for a single scene (a warp takes an equal
-  // range of the work items; with more waves a small scene's few items would
+  // range of the work items, also in small scenes: fewer CTAs make a warp take
+  // several in turn, 511 -> 524 us a pass of 21,000 particles, 831 -> 867 of
+  // 108,000; with more waves a small scene's few items would
   // wait for one another), four for a batch (the scenes' shares are whole CTAs)
   const long long GP = (long long)b->sms * p2g_resident(b->dim) * (n == 1 ? 1 : 4);
   int* Gm = b->hofs.data() + MAP_G * (n + 1);
