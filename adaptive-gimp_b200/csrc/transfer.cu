@@ -1517,7 +1517,7 @@ __device__ __forceinline__ void g2p_staged(const Ctx& c, const G2PScale& sc, int
   // weight (S) and gradient (T) first; the other axes' factors are applied
   // once per row.  (Summing planes before the first axis as well saves a third
   // of the multiply-adds, but its partial sums do not fit the 64 registers:
-  // 114 against 111 us for 1.9M particles, 34.6 against 30.7 for 300,000.)
+  // 114 against 111 us for 1.9M particles, 34.6 against 30.7 for 600,000.)
 #pragma unroll
   for (int n0 = 0; n0 < 3; ++n0) {
     float w0, g0;
@@ -1588,7 +1588,7 @@ __global__ void __launch_bounds__(CH, 1024 / CH) k_g2p(Batch B) {
   const int i = threadIdx.x;
   // The items of this CTA come 32 at a time through shared memory and a
   // particle's source slot is read one item ahead, so an item starts with the
-  // reads of its particles' rows (300,000 static particles 27.4 -> 25.3 us).
+  // reads of its particles' rows (600,000 static particles 27.4 -> 25.3 us).
   // Items of 128 particles, not 256, halve the lanes idle in a block's last
   // item (30.7 -> 27.4; 1.9M particles 111 -> 107); 64 load a tile for too few
   // (33, 138).
