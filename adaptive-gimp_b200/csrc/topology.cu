@@ -794,7 +794,7 @@ __global__ void k_bin(Batch B) {
 // latency of two dependent L2 round trips, so the rounds' loads are issued
 // together.  Two kernels before (a scan over per-bin counts, which cost k_bin a
 // second atomic per particle group, then the cells' offsets): 20,000 2D
-// particles 9.5 -> 5.4 us, 256 2D scenes 33 -> 30 us, and k_bin with 1.9M 3D
+// particles 7.7 -> 5.4 us, 256 2D scenes 33 -> 30 us, and k_bin with 1.9M 3D
 // particles 46 -> 40 us, with 15.5M 330 -> 300 us.
 template <int D>
 __global__ void __launch_bounds__(256) k_bins(Batch B) {

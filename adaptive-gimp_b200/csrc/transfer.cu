@@ -718,8 +718,7 @@ __global__ void __launch_bounds__(Stage<D>::PER) k_restrict(Batch B, int l) {
 // for a staging round trip per block to pay.  Bound by the latency of L2
 // reads: a node's masks are loaded together, then the nodes they select
 // (before, each weight's mask and then its node: 20,000 particles restriction
-// 6.7 -> 4.4 us, prolongation 5.3 -> 4.0; 256 scenes 28 -> 26 and 31, as
-// before).  Three CTAs an SM: with two the batch takes 31 us (restriction).
+// 6.7 -> 4.4 us, prolongation 5.3 -> 4.0; 256 scenes 26 and 31, as before).  Three CTAs an SM: with two the batch takes 31 us (restriction).
 template <int D>
 __global__ void __launch_bounds__(256, 3) k_restrict_gather(Batch B, int l) {
   SCENE_CTA(B, MAP_G);
