@@ -184,7 +184,7 @@ void batch_free(agimp_batch* b) {
 // when the kernel ends; with more, shorter ones the SMs fill up evenly, but
 // each wave costs some 1.5 us of prologues.  Times in us of ghost marks / bins
 // / G2P: 1.9M 3D particles, one wave 32 / 40 / 107, two 28 / 36 / 103, four 36
-// for the bins, 102 for G2P and 5 lost in the other kernels; 256 2D scenes, 5M:
+// for the bins, 102 for G2P and 5 lost in the other kernels; 256 2D scenes:
 // one 45 / 60 / 141, four 38 / 52 / 133, eight 58 for the bins and 142 for G2P;
 // 15.5M 3D: one 114 / 297 / 784, four 247 for the bins and 736 for G2P, eight 94
 // / 242 / 717; the small scenes lose 2 to 3 us a kernel from the second wave on.
