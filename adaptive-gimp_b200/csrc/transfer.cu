@@ -1148,18 +1148,36 @@ __device__ __forceinline__ bool sur_handoff(const Ctx& c, const float* U, const 
 // Snow return map of G2P's trial state F (in place): states whose singular
 // values are provably inside the clamp interval are unchanged; the others get
 // an SVD, are recorded when the recorder samples this particle, and are
-// projected exactly or handed to the surrogate.  (In 3D, G2P itself
-// projects the states near a rotation when neither recorder nor surrogate
-// wants their SVD.)
+// projected exactly or handed to the surrogate.  In 3D without a surrogate the
+// states near a rotation take snow_clamp_near, as in G2P, which lists them here
+// only for a recorder: recording changes no result, and a state that is not
+// sampled needs no SVD.
 template <int D>
 __device__ __forceinline__ void snow_return_map(const Ctx& c, float* F, float& jp, int j) {
-  if (singular_values_within<D>(F, 1.f - c.theta_c, 1.f + c.theta_s)) return;
-  float U[D * D], sg[D], V[D * D];
-  svd_d<D>(F, U, sg, V);
-  const bool dom = (c.rec_X || c.sur) && sur_domain<D>(F, sg, jp);
-  if (c.rec_X && dom && j % c.rec_stride == 0) record_pair<D>(c, sg, jp);
-  if (c.sur && dom && sur_handoff<D>(c, U, sg, V, jp, j)) return;
-  snow_clamp_rebuild<D>(c, U, sg, V, F, jp);
+  const float lo = 1.f - c.theta_c, hi = 1.f + c.theta_s;
+  bool within = singular_values_within<D>(F, lo, hi), near = false;
+  float Fn[D * D], jn = jp;
+  if constexpr (D == 3) {
+    if (c.rec_X && !c.sur) {
+#pragma unroll
+      for (int k = 0; k < D * D; ++k) Fn[k] = F[k];
+      near = snow_clamp_near(Fn, jn, lo, hi);
+      within = within || (near && j % c.rec_stride != 0);  // no SVD wanted
+    }
+  }
+  if (!within) {
+    float U[D * D], sg[D], V[D * D];
+    svd_d<D>(F, U, sg, V);
+    const bool dom = (c.rec_X || c.sur) && sur_domain<D>(F, sg, jp);
+    if (c.rec_X && dom && j % c.rec_stride == 0) record_pair<D>(c, sg, jp);
+    if (c.sur && dom && sur_handoff<D>(c, U, sg, V, jp, j)) return;
+    if (!near) snow_clamp_rebuild<D>(c, U, sg, V, F, jp);
+  }
+  if (near) {
+#pragma unroll
+    for (int k = 0; k < D * D; ++k) F[k] = Fn[k];
+    jp = jn;
+  }
 }
 
 // F and Jp of particle j of a state (the rows' other words stay as they are).
