@@ -1087,9 +1087,10 @@ __host__ __device__ __forceinline__ bool snow_clamp_near(float* F, float& jp, fl
   }
   if (k[0] == 0.f && k[1] == 0.f && k[2] == 0.f) return true;
   {
-    // jp Jo / Jn, the quotient corrected by its remainder
+    // jp Jo / Jn, the quotient corrected by its remainder (an infinite one has none)
     const float a = jp * Jo, r = divide_fast(1.f, Jn), q = a * r;
-    jp = fmaf(r, fmaf(-q, Jn, a), q);
+    const float rem = fmaf(-q, Jn, a);
+    jp = rem == rem ? fmaf(r, rem, q) : q;
   }
   float K[6];  // as E
 #pragma unroll

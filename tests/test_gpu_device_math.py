@@ -165,3 +165,11 @@ def test_snow_refuses_far_and_inverted(snow):
     assert not ok.any()
     np.testing.assert_array_equal(got, far.astype(np.float32))
     assert (jp == 1.25).all()
+
+
+@pytest.mark.parametrize("jp0", [float("inf"), float("-inf"), 0.0])
+def test_snow_ratio_without_a_remainder(snow, jp0):
+    F = np.tile(np.diag([1.1, 1.0, 1.0]), (3, 1, 1))
+    got, jp, ok = _near(snow, F, jp0)
+    assert ok.all()
+    np.testing.assert_array_equal(jp, np.float32(jp0))
