@@ -294,7 +294,7 @@ agimp_status agimp_create(const agimp_params* p, int32_t device, agimp_sim** out
   if (!p || !out) return AGIMP_INVALID_ARG;
   *out = nullptr;
   if ((p->dim != 2 && p->dim != 3) || p->level < 1 || p->level > MAXL || p->coarsest_size < 4 ||
-      (p->coarsest_size & (p->coarsest_size - 1)) || p->n_particles < 0 || p->n_particles > (int64_t)1 << 30 ||
+      (p->coarsest_size & (p->coarsest_size - 1)) || p->n_particles < 0 || p->n_particles > MAX_PARTICLES ||
       p->n_colliders < 0 || p->n_colliders > 4 || !(p->radius > 0.0 && p->radius <= 0.5) ||
       (p->coarsest_size << (p->level - 1)) > (1 << 13) || p->plasticity < 0 || p->plasticity > 1 ||
       p->invalid_nodes < 0 || p->invalid_nodes > 1)

@@ -40,6 +40,11 @@ constexpr int P2G_TASKS = 10, P2G_LOG_TMAX = 3;
 __host__ __device__ constexpr int p2g_log_task(int per_cell, int n) {
   return per_cell <= 4 || n < 150000 ? 2 : P2G_LOG_TMAX;
 }
+// A work item holds its place among the bin's items in 24 bits.  Tasks below the
+// longest come in bins of at most 5 particles a cell or in scenes of less than
+// 150,000, so a place beyond needs more particles than a simulator takes.
+constexpr long long MAX_PARTICLES = 1ll << 30;
+static_assert(MAX_PARTICLES / (P2G_TASKS << P2G_LOG_TMAX) + 64 < 1ll << 24, "item of the bin");
 
 enum : uint32_t { ACT = 1u, GHO = 2u, TJ = 4u, CUL = 8u };
 enum : uint32_t { ERR_OOB = 1u, ERR_ESCAPED = 2u, ERR_MAP_OOB = 4u, ERR_NOBIN = 8u, ERR_MLP = 16u };

@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(256) k_bins(Batch B) {
       for (int k = sub; k * CH < total[r]; k += LANES)
         c.chunks[c0 + k] = make_int4(l, blk, p0 + k * CH, min(CH, total[r] - k * CH));
       for (int k = sub; k * P2G_TASKS < tasks[r]; k += LANES)
-        c.items[i0 + k] = make_int4(l | (log_task[r] << 4) | (k << 8), blk, b, p0 + total[r]);
+        c.items[i0 + k] = make_int4(l | (log_task[r] << 4) | (int)((unsigned)k << 8), blk, b, p0 + total[r]);
       p0 += total[r];
       c0 += (total[r] + CH - 1) / CH;
       i0 += (tasks[r] + P2G_TASKS - 1) / P2G_TASKS;

@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(32 * P2GLayout<D>::WARPS, P2GLayout<D>::CTAS) 
   int bin = -1, excl = 0, nt0 = 0, off0 = 0, off1 = 0, c0 = 0, c1 = 0, tasks = 0;
   int4 it = c.items[i0];
   for (int i = i0; i < i1; ++i) {
-    const int l = it.x & 15, lt = (it.x >> 4) & 15, first = (it.x >> 8) * Y::TASKS, blk = it.y;
+    const int l = it.x & 15, lt = (it.x >> 4) & 15, first = (int)((unsigned)it.x >> 8) * Y::TASKS, blk = it.y;
     if (it.z != bin) {
       // the bin's cells: lane holds cells 2 lane, 2 lane + 1 (3D) or cell
       // lane (2D): their particles, and the tasks of the cells before them
