@@ -33,24 +33,32 @@ Ctx& sim_ctx(agimp_sim* s) {
   return s->c;
 }
 
-// Grid-stride CTAs per SM before any tuning, by the particles of all scenes.  A
-// kernel of a small scene ends with its slowest chain of dependent reads, and
-// launching CTAs with nothing to do delays it by about 1 us per 1184; a larger
-// scene needs the warps.  Whole passes in us at 8 / 6 / 4 / 2 per SM: 21,000
-// particles (static 2D) 556 / 537 / 515 / 500, 27,000 (dynamic 2D) 740 / 731 /
-// 706 / 706, 81,000 (3D sphere) 594 / 554 / 549 / 563, 108,000 (dynamic 2D) 837
-// / 829 / 813 / 878, 195,000 (static 3D) 445 / 436 / 452 / 524, 316,000 (3D
-// sphere) 815 / 796 / 824 / 956, 358,000 (static 3D) 578 / 580 / 623 / 744.
-static int default_ctas(long long particles) {
-  return particles <= 32768 ? 2 : particles <= 131072 ? 4 : particles <= 327680 ? 6 : 8;
+// Grid-stride CTAs per SM before any tuning, by the particles and stored lattice
+// elements of all scenes.  A kernel of a small compact scene ends with its
+// slowest chain of dependent reads, and launching CTAs with nothing to do delays
+// it by about 1 us per 1184.  But half of the kernels sweep the active blocks,
+// which the host does not know: scattered particles touch many each (30,000 in
+// 3D 243,000 blocks, as a body 344) and need the warps.  Substeps in us at 8 /
+// 6 / 4 / 2 per SM: scattered on three levels, 10,000 3D particles 942 / 943 /
+// 1134 / 1475, 100,000 1925 / 2008 / 2417 / 3296, 30,000 2D 165 / 169 / 170 /
+// 204; bodies of 80,000 3D 89 / - / 83 / 85, 30,000 2D 56 / - / 54 / 53.
+static int default_ctas(int dim, int sms, long long particles, long long elements) {
+  int n = particles > 327680 ? 8 : dim == 3 || particles > 131072 ? 6 : 4;
+  // no more than a thread per element, which nothing can use
+  const long long all = std::max(particles, elements), per = 256ll * sms;
+  if (all < n * per) n = std::max(2, (int)((all + per - 1) / per));
+  return n;
 }
 
 agimp_status batch_init(agimp_batch* b) {
   const int n = (int)b->sims.size();
   {
-    long long sumN = 0;
-    for (agimp_sim* s : b->sims) sumN += s->c.N;
-    b->tune.ctas_per_sm = default_ctas(sumN);
+    long long sumN = 0, elements = 0;
+    for (agimp_sim* s : b->sims) {
+      sumN += s->c.N;
+      for (int l = 0; l < s->c.L; ++l) elements += s->c.lev[l].nblocks << (2 * s->c.dim);
+    }
+    b->tune.ctas_per_sm = default_ctas(b->sims[0]->c.dim, b->sims[0]->c.sms, sumN, elements);
   }
   {
     const char* e = std::getenv("AGIMP_PDL");
