@@ -66,6 +66,12 @@ class Tuning(ctypes.Structure):
         return dict(chunk=self.chunk, ctas_per_sm=self.ctas_per_sm, ms_per_substep=self.ms_per_substep)
 
 
+def tuning_of(now, chunk, ctas_per_sm):
+    """The launch tuning with the given values, None taken from the present one."""
+    return Tuning(int(now["chunk"] if chunk is None else chunk),
+                  int(now["ctas_per_sm"] if ctas_per_sm is None else ctas_per_sm), 0.0)
+
+
 SHAPE_BOX = 0
 SHAPE_SPHERE = 1
 

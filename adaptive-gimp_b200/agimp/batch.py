@@ -54,8 +54,9 @@ class SceneBatch:
         _capi.check(self._L.agimp_batch_get_tuning(self._h, ctypes.byref(t)), self._h, "get tuning", batch=True)
         return t.as_dict()
 
-    def set_tuning(self, chunk=256, ctas_per_sm=8):
-        t = _capi.Tuning(int(chunk), int(ctas_per_sm), 0.0)
+    def set_tuning(self, chunk=None, ctas_per_sm=None):
+        """3D G2P work-item size (64, 128, 256, 512) and grid-stride CTAs per SM; None keeps the present one."""
+        t = _capi.tuning_of(self.tuning, chunk, ctas_per_sm)
         _capi.check(self._L.agimp_batch_set_tuning(self._h, ctypes.byref(t)), self._h, "set tuning", batch=True)
 
     def autotune(self, dt0, trials=5, stream=None):

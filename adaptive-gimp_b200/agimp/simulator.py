@@ -430,9 +430,9 @@ class AdaptiveGIMP:
         _capi.check(self._L.agimp_get_tuning(self._h, ctypes.byref(t)), self._h, "get tuning")
         return t.as_dict()
 
-    def set_tuning(self, chunk=256, ctas_per_sm=8):
-        """3D G2P work-item size (64, 128, 256, 512) and grid-stride CTAs per SM."""
-        t = _capi.Tuning(int(chunk), int(ctas_per_sm), 0.0)
+    def set_tuning(self, chunk=None, ctas_per_sm=None):
+        """3D G2P work-item size (64, 128, 256, 512) and grid-stride CTAs per SM; None keeps the present one."""
+        t = _capi.tuning_of(self.tuning, chunk, ctas_per_sm)
         _capi.check(self._L.agimp_set_tuning(self._h, ctypes.byref(t)), self._h, "set tuning")
 
     def autotune(self, dt0, trials=5, stream=None):

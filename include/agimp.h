@@ -340,10 +340,12 @@ typedef struct agimp_tuning {
 } agimp_tuning;
 agimp_status agimp_set_tuning(agimp_sim* s, const agimp_tuning* t);
 agimp_status agimp_get_tuning(const agimp_sim* s, agimp_tuning* t);
-/* Measure every (chunk, ctas_per_sm) in {64, 128, 256, 512} x {2, 4, 8, 16}:
+/* Measure the present tuning and every (chunk, ctas_per_sm) in {64, 128, 256,
+ * 512} x {2, 4, 8, 16} (2D, where chunk changes no launch: the present chunk):
  * two warm-up and `trials` timed substeps each, all from the current state,
  * which is restored afterwards (the simulation does not advance).  Keeps and
- * returns the fastest.  Synchronizes the stream. */
+ * returns the fastest; the present tuning only where it beats the others by 2
+ * percent.  Synchronizes the stream. */
 agimp_status agimp_autotune(agimp_sim* s, float dt, int32_t trials, agimp_tuning* best, void* stream);
 
 /* ---- Batches (no counterpart in the reference).  Independent simulators on
