@@ -25,7 +25,7 @@ EXPORTS = (
     "agimp_abi_version", "agimp_status_string", "agimp_default_params", "agimp_create", "agimp_destroy",
     "agimp_last_error", "agimp_set_particles", "agimp_get_particles", "agimp_set_level_map",
     "agimp_clear_level_map", "agimp_get_bins", "agimp_substep", "agimp_set_graphs", "agimp_refine_levels", "agimp_get_grid",
-    "agimp_get_node_mask", "agimp_errors", "agimp_get_stats", "agimp_kernels_per_substep",
+    "agimp_get_node_mask", "agimp_errors", "agimp_get_stats", "agimp_kernels_per_substep", "agimp_launches_per_substep",
     "agimp_profile_substep", "agimp_refine_levels_noalloc",
     "agimp_mlp_num_params", "agimp_mlp_create", "agimp_mlp_destroy", "agimp_mlp_set_params", "agimp_mlp_get_params",
     "agimp_mlp_forward", "agimp_mlp_errors", "agimp_wait_selftest", "agimp_mlp_grad", "agimp_mlp_train_step", "agimp_mlp_reset_optimizer",
@@ -33,7 +33,7 @@ EXPORTS = (
     "agimp_set_tuning", "agimp_get_tuning", "agimp_autotune",
     "agimp_batch_create", "agimp_batch_destroy", "agimp_batch_last_error", "agimp_batch_substep",
     "agimp_batch_set_graphs", "agimp_batch_set_tuning", "agimp_batch_get_tuning", "agimp_batch_autotune",
-    "agimp_batch_kernels_per_substep", "agimp_batch_profile_substep", "agimp_batch_set_surrogate",
+    "agimp_batch_kernels_per_substep", "agimp_batch_launches_per_substep", "agimp_batch_profile_substep", "agimp_batch_set_surrogate",
     "agimp_batch_surrogate_stats",
     "agimp_render_mask", "agimp_render_particles", "agimp_get_particles_async", "agimp_batch_positions_async",
     "agimp_batch_set_particles",
@@ -140,6 +140,8 @@ def load(path: str | None = None):
     L.agimp_get_bins.argtypes = [vp, vp, ctypes.c_int32, vp]
     L.agimp_kernels_per_substep.argtypes = [vp]
     L.agimp_kernels_per_substep.restype = ctypes.c_int32
+    L.agimp_launches_per_substep.argtypes = [vp]
+    L.agimp_launches_per_substep.restype = ctypes.c_int32
     L.agimp_profile_substep.argtypes = [vp, ctypes.c_float, fp, ctypes.c_int32, vp]
     L.agimp_refine_levels_noalloc.argtypes = [vp, ctypes.c_int64, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32,
                                               ctypes.c_int32, vp, vp]
@@ -175,6 +177,8 @@ def load(path: str | None = None):
     L.agimp_batch_autotune.argtypes = [vp, ctypes.c_float, ctypes.c_int32, tp, vp]
     L.agimp_batch_kernels_per_substep.argtypes = [vp]
     L.agimp_batch_kernels_per_substep.restype = ctypes.c_int32
+    L.agimp_batch_launches_per_substep.argtypes = [vp]
+    L.agimp_batch_launches_per_substep.restype = ctypes.c_int32
     L.agimp_batch_profile_substep.argtypes = [vp, ctypes.c_float, fp, ctypes.c_int32, vp]
     L.agimp_get_particles_async.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     L.agimp_batch_positions_async.argtypes = [vp, vp, vp]

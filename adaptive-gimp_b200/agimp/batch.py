@@ -121,7 +121,12 @@ class SceneBatch:
         # argument order of the C entry point: x, v, F, C, m, g, Jp
         _capi.check(self._L.agimp_batch_set_particles(self._h, *args, mem, st), self._h, "batch upload", batch=True)
 
+    def launches_per_substep(self):
+        """Kernels one substep launches for the whole batch."""
+        return int(self._L.agimp_batch_launches_per_substep(self._h))
+
     def kernels_per_substep(self):
+        """Passes of one substep without the batch's surrogate; the two over the bins' offsets share a kernel."""
         return int(self._L.agimp_batch_kernels_per_substep(self._h))
 
     # -- surrogate return map over the batch (extension) ------------------------

@@ -451,7 +451,12 @@ class AdaptiveGIMP:
         _capi.check(self._L.agimp_profile_substep(self._h, float(dt0), ms, len(ms), st), self._h, "profile")
         return dict(zip(_capi.PHASES, list(ms)))
 
+    def launches_per_substep(self):
+        """Kernels one substep launches."""
+        return int(self._L.agimp_launches_per_substep(self._h))
+
     def kernels_per_substep(self):
+        """Passes of one substep: launches_per_substep() and one, since the two over the bins' offsets share a kernel."""
         return int(self._L.agimp_kernels_per_substep(self._h))
 
     # -- predicates (adaptive_gimp.py:126-140), vectorised over I[..., dim] --

@@ -606,11 +606,18 @@ void wait_readback(agimp_sim* s, int buf, cudaStream_t use) {
   }
 }
 
-int batch_kernels(agimp_batch* b) {
-  const BatchLaunch bl = make_launch(b, 0);
+// the surrogate's kernels of a single simulator's substep
+static int single_surrogate(const agimp_batch* b) {
   const Ctx& c = b->sims[0]->c;
-  return kernels_per_substep(bl) + ((b->single && c.sur && c.plast == 1 && c.N) ? 2 : 0);
+  return (b->single && c.sur && c.plast == 1 && c.N) ? 2 : 0;
 }
+
+int batch_launches(agimp_batch* b) {
+  const BatchLaunch bl = make_launch(b, 0);
+  return launches_per_substep(bl) + (b->single ? single_surrogate(b) : bl.sur ? 2 : 0);
+}
+
+int batch_kernels(agimp_batch* b) { return launches_per_substep(make_launch(b, 0)) + 1 + single_surrogate(b); }
 
 agimp_status batch_set_tuning(agimp_batch* b, const agimp_tuning* t) {
   if (!t || (t->chunk != 64 && t->chunk != 128 && t->chunk != 256 && t->chunk != 512) || t->ctas_per_sm < 1 ||

@@ -809,6 +809,8 @@ agimp_status agimp_get_stats(agimp_sim* s, agimp_stats* out) {
   return AGIMP_OK;
 }
 
+int32_t agimp_launches_per_substep(const agimp_sim* s) { return s ? batch_launches(s->self) : 0; }
+
 int32_t agimp_kernels_per_substep(const agimp_sim* s) {
   if (!s) return 0;
   return batch_kernels(s->self);
@@ -1094,6 +1096,10 @@ agimp_status agimp_batch_surrogate_stats(agimp_batch* b, int64_t* handed, int64_
   if (rejected) *rejected = rej;
   if (errors) *errors = h[1] ? AGIMP_ERR_WAIT : 0u;
   return AGIMP_OK;
+}
+
+int32_t agimp_batch_launches_per_substep(const agimp_batch* b) {
+  return b ? batch_launches(const_cast<agimp_batch*>(b)) : 0;
 }
 
 int32_t agimp_batch_kernels_per_substep(const agimp_batch* b) {

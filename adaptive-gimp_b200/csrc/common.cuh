@@ -1289,6 +1289,6 @@ int p2g_resident(int dim);  // k_p2g CTAs an SM holds at once
 // surrogate MLP forward over a device-side sample count (mlp.cu)
 void launch_mlp_forward_dev(const void* packed, const float* P, const float* X, float* Y, const int32_t* n_dev,
                             long long cap, int32_t* err, int sms, cudaStream_t s);
-int kernels_per_substep(const BatchLaunch& bl);
+int launches_per_substep(const BatchLaunch& bl);  // without the surrogate's
 
 }  // namespace agimp

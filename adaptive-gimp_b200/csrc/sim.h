@@ -136,6 +136,7 @@ void batch_drop_graphs(agimp_batch* b);
 // n substeps of every scene on `use`; with ev, one substep with phase events
 // and no graph.
 agimp_status batch_step(agimp_batch* b, float dt, int n, cudaStream_t use, cudaEvent_t* ev);
+int batch_launches(agimp_batch* b);
 int batch_kernels(agimp_batch* b);
 agimp_status batch_positions_async(agimp_batch* b, float* x, cudaStream_t use);
 agimp_status batch_set_particles(agimp_batch* b, const float* x, const float* v, const float* F, const float* C,

@@ -957,10 +957,11 @@ void launch_substep(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   }
 }
 
-// passes of a substep: a kernel each, but for the two of the bins' offsets
-// (particles per bin, cells inside it), which share k_bins
-int kernels_per_substep(const BatchLaunch& bl) {
-  const int topo = 10 - (bl.any_dynamic ? 0 : 1) + (bl.dim == 3 && bl.maxL > 1 ? 1 : 0);
+// kernels of a substep: nine of run_topology (k_mark_hier only with a dynamic
+// scene, k_level_masks only in 3D with several levels), P2G, G2P, the return map,
+// and the grid operation or the transfers between the levels
+int launches_per_substep(const BatchLaunch& bl) {
+  const int topo = 9 - (bl.any_dynamic ? 0 : 1) + (bl.dim == 3 && bl.maxL > 1 ? 1 : 0);
   return topo + 2 + (bl.maxL == 1 ? 1 : 0) + (bl.any_plastic ? 1 : 0) + 2 * (bl.maxL - 1);
 }
 

@@ -461,7 +461,7 @@ def run_agimp(a):
             "algorithmic_bytes": dom_bytes,
             "p2g_g2p_combined_frac": (nb * (b_p2g + b_g2p) / ((phases["p2g"] + phases["g2p"]) / 1e3) / 1e9) / hbm}
     n_refines = sum(1 for i in range(a.warmup, a.warmup + a.steps) if scene.refine_every and i % scene.refine_every == 0)
-    launches = a.steps * (sim.kernels_per_substep() - 1) + n_refines * refine_kernels(scene)
+    launches = a.steps * sim.launches_per_substep() + n_refines * refine_kernels(scene)
     out = {
         "metric": METRIC, "value": value, "unit": METRIC, "n_gpus": world, "steps": a.steps, "warmup": a.warmup,
         "ms_per_step": ms_max / a.steps, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
@@ -626,7 +626,7 @@ def run_batch(a):
                                                       "unit": "domain lengths"}},
         "roofline": roof,
         "phases_ms": phases,
-        "gpu_launches": a.steps * (batch.kernels_per_substep() - 1),
+        "gpu_launches": a.steps * batch.launches_per_substep(),
         "clocks": clk.summary(),
         "device_errors": int(np.bitwise_or.reduce(errors)),
     }

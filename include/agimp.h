@@ -196,8 +196,11 @@ agimp_status agimp_get_node_mask(agimp_sim* s, int32_t* out, int32_t memory, voi
 agimp_status agimp_errors(agimp_sim* s, uint32_t* bits, int32_t clear);
 agimp_status agimp_get_stats(agimp_sim* s, agimp_stats* out);
 
-/* Number of passes of one substep (for launch accounting): a kernel each, but
- * for the two passes over the bins' offsets, which are one launch. */
+/* Number of kernels one substep launches, the surrogate's included. */
+int32_t agimp_launches_per_substep(const agimp_sim* s);
+/* Number of passes of one substep: a kernel each, but for the two passes over
+ * the bins' offsets, which share one.  Not a count of launches, which is
+ * agimp_launches_per_substep. */
 int32_t agimp_kernels_per_substep(const agimp_sim* s);
 
 /* One substep with direct launches and CUDA events between its phases;
@@ -368,6 +371,9 @@ agimp_status agimp_batch_set_tuning(agimp_batch* b, const agimp_tuning* t);
 agimp_status agimp_batch_get_tuning(const agimp_batch* b, agimp_tuning* t);
 /* As agimp_autotune, over the whole batch. */
 agimp_status agimp_batch_autotune(agimp_batch* b, float dt, int32_t trials, agimp_tuning* best, void* stream);
+/* As agimp_launches_per_substep and agimp_kernels_per_substep; a batch's own
+ * surrogate is only in the former. */
+int32_t agimp_batch_launches_per_substep(const agimp_batch* b);
 int32_t agimp_batch_kernels_per_substep(const agimp_batch* b);
 /* Positions of all scenes in one copy: x [sum of N][dim] in HOST memory
  * (pinned, for overlap), scene after scene in batch order, each scene in its
