@@ -28,7 +28,6 @@ namespace agimp {
 
 constexpr int MAXL = 8;
 constexpr int CHUNK = 128;      // default G2P work item (particles of one bin) = 3D G2P CTA size
-constexpr int MAX_CHUNK = 512;  // largest work item the tuning may choose
 constexpr int MIN_CHUNK = 64;   // smallest work item (sizes the work-item buffer)
 constexpr int HALO = 4;
 
@@ -396,14 +395,6 @@ struct Corners {
   }
 };
 
-template <int D>
-__device__ __forceinline__ long long block_of(const LevelDev& V, const int* I) {
-  unsigned b = 0;
-#pragma unroll
-  for (int d = 0; d < D; ++d) b = b * (unsigned)V.nb + ((unsigned)(I[d] + HALO) >> 2);
-  return (long long)b;
-}
-
 // element coordinates of local index `loc` in stored block `blk`
 template <int D>
 __device__ __forceinline__ void elem_coords(const LevelDev& V, long long blk, int loc, int* I) {
@@ -445,19 +436,6 @@ __device__ __forceinline__ uint32_t* nm_word(const Ctx& c, int l, const int* I) 
     in = in && P[d] >= 0 && P[d] <= c.sz;
   }
   return in ? &c.nmask[elem_of<D>(c.lev[c.L - 1], P)] : nullptr;
-}
-
-template <int D>
-__device__ __forceinline__ void nm_or(const Ctx& c, int l, const int* I, uint32_t bits) {
-  const int s = c.L - 1 - l;
-  int P[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) {
-    P[d] = I[d] * (1 << s);
-    if (P[d] < 0 || P[d] > c.sz) return;  // unobservable: never read by a predicate
-  }
-  uint32_t* w = &c.nmask[elem_of<D>(c.lev[c.L - 1], P)];
-  if ((*w & bits) != bits) atomicOr(w, bits);
 }
 
 __device__ __forceinline__ bool is_valid(uint32_t nm) { return nm > 0u; }
@@ -581,8 +559,6 @@ __device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
 // the same on float2 operands
 __device__ __forceinline__ f2 pk2(float2 a) { return f2_make(a.x, a.y); }
 __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c) { return f2_get(f2_fma(pk2(a), pk2(b), pk2(c))); }
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b) { return f2_get(f2_mul(pk2(a), pk2(b))); }
-__device__ __forceinline__ float2 fadd2(float2 a, float2 b) { return f2_get(f2_add(pk2(a), pk2(b))); }
 __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 #endif
 

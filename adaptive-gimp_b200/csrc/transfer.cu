@@ -718,9 +718,11 @@ __global__ void __launch_bounds__(Stage<D>::PER) k_restrict(Batch B, int l) {
 // for a staging round trip per block to pay.  Bound by the latency of L2
 // reads: a node's masks are loaded together, then the nodes they select
 // (before, each weight's mask and then its node: 20,000 particles restriction
-// 6.7 -> 4.4 us, prolongation 5.3 -> 4.0; 256 scenes 26 and 31, as before).  Three CTAs an SM: with two the batch takes 31 us (restriction).
+// 6.7 -> 4.4 us, prolongation 5.3 -> 4.0; 256 scenes 26 and 31, as before).
+// Three CTAs an SM: with two the batch's restriction takes 31 us.
 template <int D>
 __global__ void __launch_bounds__(256, 3) k_restrict_gather(Batch B, int l) {
+  static_assert(D == 2, "3D transfers are staged");
   SCENE_CTA(B, MAP_G);
   const bool restrict_l = l < c.L;
   if (!restrict_l && l != 1) return;
@@ -743,53 +745,49 @@ __global__ void __launch_bounds__(256, 3) k_restrict_gather(Batch B, int l) {
     bool any = false;
     if (restrict_l && is_valid(cm)) {
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      // nine sources at a time (all in 2D, a plane in 3D): their masks are read
-      // together, then the nodes that count (two memory latencies)
+      // the nine sources' masks are read together, then the nodes that count (two
+      // memory latencies)
+      unsigned fidx[9], use = 0;
+      uint32_t nm[9];
+      auto weight = [&](int a, int* I) {  // source a's node and weight
+        int nrm = 0;
 #pragma unroll
-      for (int a0 = 0; a0 < ((D == 2) ? 9 : 27); a0 += 9) {
-        unsigned fidx[9], use = 0;
-        uint32_t nm[9];
-        auto weight = [&](int a, int* I) {  // source a's node and weight
-          int nrm = 0;
-#pragma unroll
-          for (int d = D - 1; d >= 0; --d) {
-            const int dI = a % 3 - 1;
-            a /= 3;
-            I[d] = 2 * K[d] - dI;
-            nrm += dI != 0;
-          }
-          return (nrm == 0) ? 1.f : (nrm == 1) ? 0.5f : (nrm == 2) ? 0.25f : 0.125f;
-        };
-#pragma unroll
-        for (int a = 0; a < 9; ++a) {
-          int I[D];
-          weight(a0 + a, I);
-          bool ok = true;
-#pragma unroll
-          for (int d = 0; d < D; ++d) ok = ok && I[d] >= 0 && I[d] <= lsz;
-          fidx[a] = (unsigned)elem_of<D>(Vf, I);
-          nm[a] = ok ? level_mask<D>(c, l, I, fidx[a]) : 0u;
+        for (int d = D - 1; d >= 0; --d) {
+          const int dI = a % 3 - 1;
+          a /= 3;
+          I[d] = 2 * K[d] - dI;
+          nrm += dI != 0;
         }
-        float4 f[9];
+        return (nrm == 0) ? 1.f : (nrm == 1) ? 0.5f : 0.25f;
+      };
 #pragma unroll
-        for (int a = 0; a < 9; ++a) {
-          int I[D];
-          if ((is_activated(nm[a]) && weight(a0 + a, I) == 1.f) || is_tj(nm[a]) || is_ghost(nm[a])) {
-            f[a] = Vf.node[fidx[a]];
-            use |= 1u << a;
-          }
-        }
-        any = any || use;
+      for (int a = 0; a < 9; ++a) {
+        int I[D];
+        weight(a, I);
+        bool ok = true;
 #pragma unroll
-        for (int a = 0; a < 9; ++a) {
-          if (!(use >> a & 1u)) continue;
-          int I[D];
-          const float w = weight(a0 + a, I);
-          acc.x += f[a].x * w;
-          acc.y += f[a].y * w;
-          if (D == 3) acc.z += f[a].z * w;
-          acc.w += f[a].w * w;
+        for (int d = 0; d < D; ++d) ok = ok && I[d] >= 0 && I[d] <= lsz;
+        fidx[a] = (unsigned)elem_of<D>(Vf, I);
+        nm[a] = ok ? level_mask<D>(c, l, I, fidx[a]) : 0u;
+      }
+      float4 f[9];
+#pragma unroll
+      for (int a = 0; a < 9; ++a) {
+        int I[D];
+        if ((is_activated(nm[a]) && weight(a, I) == 1.f) || is_tj(nm[a]) || is_ghost(nm[a])) {
+          f[a] = Vf.node[fidx[a]];
+          use |= 1u << a;
         }
+      }
+      any = use != 0;
+#pragma unroll
+      for (int a = 0; a < 9; ++a) {
+        if (!(use >> a & 1u)) continue;
+        int I[D];
+        const float w = weight(a, I);
+        acc.x += f[a].x * w;
+        acc.y += f[a].y * w;
+        acc.w += f[a].w * w;
       }
       if (any) o = make_float4(o.x + acc.x, o.y + acc.y, o.z + acc.z, o.w + acc.w);
     }
@@ -802,6 +800,7 @@ __global__ void __launch_bounds__(256, 3) k_restrict_gather(Batch B, int l) {
 
 template <int D>
 __global__ void k_prolong_gather(Batch B, int l) {
+  static_assert(D == 2, "3D transfers are staged");
   SCENE_CTA(B, MAP_G);
   if (l >= c.L) return;
   const LevelDev& Vc = c.lev[l - 1];
@@ -849,22 +848,21 @@ __global__ void k_prolong_gather(Batch B, int l) {
     float4 o = gridop_value<D>(c, l, J, nm, nd);
     if (tg || even) {
       const bool take = tg || is_activated(nm);  // (an even node's only source is a = 0)
-      const float w = (nodd == 0) ? 1.f : (nodd == 1) ? 0.5f : (nodd == 2) ? 0.25f : 0.125f;
+      const float w = (nodd == 0) ? 1.f : (nodd == 1) ? 0.5f : 0.25f;
       float4 cv[1 << D];
 #pragma unroll
       for (int a = 0; a < (1 << D); ++a)
         if (take && is_valid(cm[a])) cv[a] = Vc.node[cidx[a]];
-      float acc[3] = {0.f, 0.f, 0.f};
+      float acc[2] = {0.f, 0.f};
 #pragma unroll
       for (int a = 0; a < (1 << D); ++a)
         if (take && is_valid(cm[a])) {
           acc[0] += cv[a].x * w;
           acc[1] += cv[a].y * w;
-          if (D == 3) acc[2] += cv[a].z * w;
         }
       o.x = acc[0];
       o.y = acc[1];
-      o.z = acc[2];
+      o.z = 0.f;
     }
     Vf.node[fidx] = o;
   }
@@ -1740,7 +1738,7 @@ void launch_transfer(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   // the first launch after the join is a plain one
   bool first = true;
   for (int l = bl.maxL - 1; l >= 1; --l, first = false) {
-    if (staged_transfers<D>())
+    if constexpr (staged_transfers<D>())
       launch_k(pdl && !(first && bl.side), k_restrict<D>, bl.nct[MAP_T], Stage<D>::PER, 0, s, bl.b, l);
     else
       launch_k(pdl && !(first && bl.side), k_restrict_gather<D>, G, 256, 0, s, bl.b, l);
@@ -1751,7 +1749,7 @@ void launch_transfer(const BatchLaunch& bl, cudaStream_t s, cudaEvent_t* ev) {
   if (bl.maxL == 1) launch_k(pdl && !bl.side, k_gridop<D>, G, 256, 0, s, bl.b);
   if (ev) cudaEventRecord(ev[6], s);
   for (int l = 1; l < bl.maxL; ++l) {
-    if (staged_transfers<D>())
+    if constexpr (staged_transfers<D>())
       launch_k(pdl, k_prolong<D>, bl.nct[MAP_T], Stage<D>::PER, 0, s, bl.b, l);
     else
       launch_k(pdl, k_prolong_gather<D>, G, 256, 0, s, bl.b, l);
