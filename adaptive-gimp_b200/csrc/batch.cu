@@ -36,18 +36,20 @@ Ctx& sim_ctx(agimp_sim* s) {
 // Grid-stride CTAs per SM before any tuning, by the particles and stored lattice
 // elements of all scenes.  A kernel of a small compact scene ends with its
 // slowest chain of dependent reads, and launching CTAs with nothing to do delays
-// it by about 1 us per 1184.  But half of the kernels sweep the active blocks,
-// which the host does not know: scattered particles touch many each (30,000 in
-// 3D 243,000 blocks, as a body 344) and need the warps.  Substeps in us at 8 /
-// 6 / 4 / 2 per SM: scattered on three levels, 10,000 3D particles 942 / 943 /
-// 1134 / 1475, 100,000 1925 / 2008 / 2417 / 3296, 30,000 2D 165 / 169 / 170 /
-// 204; bodies of 80,000 3D 89 / - / 83 / 85, 30,000 2D 56 / - / 54 / 53.
+// it by about 1 us per 1184; a larger scene needs the warps.  Half of the kernels
+// sweep the active blocks, which the host does not know: scattered particles
+// touch many each (30,000 in 3D 243,000 blocks, as a body 344), so where the
+// lattice has room for them 3D keeps 6 and 2D 4.  Substeps in us at 8 / 6 / 4 / 2
+// per SM: scattered on three levels, 10,000 3D particles in 256^3 942 / 943 / 1134
+// / 1475, in 64^3 - / 115 / 119 / 143, 100,000 in 256^3 1925 / 2008 / 2417 / 3296,
+// 30,000 2D in 1024^2 165 / 169 / 170 / 204, in 256^2 - / - / 62 / 63; bodies of
+// 80,000 3D 89 / - / 83 / 85, 50,000 82 / 75 / 73 / 73, 30,000 2D 56 / - / 54 / 53.
 static int default_ctas(int dim, int sms, long long particles, long long elements) {
-  int n = particles > 327680 ? 8 : dim == 3 || particles > 131072 ? 6 : 4;
-  // no more than a thread per element, which nothing can use
-  const long long all = std::max(particles, elements), per = 256ll * sms;
-  if (all < n * per) n = std::max(2, (int)((all + per - 1) / per));
-  return n;
+  const int body = particles <= 32768 ? 2 : particles <= 131072 ? 4 : particles <= 327680 ? 6 : 8;
+  // a thread for two elements of a 2D lattice, for four of a 3D one (most of a
+  // touched block of 64 are far from its particle)
+  const long long span = 256ll * sms * (dim == 3 ? 4 : 2);
+  return std::max(body, (int)std::min<long long>(dim == 3 ? 6 : 4, (elements + span - 1) / span));
 }
 
 agimp_status batch_init(agimp_batch* b) {
