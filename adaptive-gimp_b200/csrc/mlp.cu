@@ -38,8 +38,8 @@ constexpr int THREADS = 256;
 // The activations are bound by the special-function unit (an exponential and a
 // reciprocal each, 16 a cycle and SM) and by the instructions around it.  For
 // |z| < 40 two of them share one reciprocal, 1 / d0 = d1 (1 / (d0 d1)), and the
-// quotients are those of a rounded division all the same (checked against it:
-// the last bit differs for one operand in 10^8): a Newton step on the
+// quotients are those of a rounded division all the same (but for less than one
+// operand in 2^20, whose last bit differs): a Newton step on the
 // reciprocal, then the quotient corrected by its remainder in fused
 // multiply-adds (P. Markstein, "Computation of elementary functions on the IBM
 // RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), two at a time.
@@ -152,9 +152,11 @@ __device__ __forceinline__ void hidden_epilogue(uint32_t taddr, const float* bia
 
 // Y[n][4] = MLP(X[n][7]) for n < N.
 //
-// What bounds it: the activations' special-function operations (silu8) and
-// the instructions around them; the products are far too thin to matter (2
-// percent of the tensor pipe).  The activations are written as packed 16-byte
+// What bounds it: the activations' special-function operations (silu8) and the
+// instructions around them, each at half of its rate, and the chain of product,
+// wait, epilogue and barrier, which 26 warps an SM overlap in part; the products
+// are far too thin to matter (7 percent of the tensor pipe).  2M rows take 173
+// us.  The activations are written as packed 16-byte
 // core-matrix rows; element by element (2-byte stores with 4-way bank
 // conflicts) and with general divisions 2M rows took 357 us.
 __global__ void __launch_bounds__(THREADS, 4) k_forward(const float* __restrict__ X, float* __restrict__ Y, long long N,
@@ -278,8 +280,8 @@ __global__ void __launch_bounds__(THREADS, 4) k_forward(const float* __restrict_
 //
 // What bounds it: the chain of six products and epilogues per tile, at two CTAs
 // per SM.  The activations stay in registers between forward and backward, and
-// no transposed copies are written (one CTA of 128 threads per SM wrote every
-// activation twice, element by element: 65,536 rows took 114 us).
+// no transposed copies are written (before, one CTA of 128 threads per SM wrote
+// every activation twice, element by element).  A call over 65,536 rows 124 -> 30 us.
 constexpr int HW = H + 8;  // width of the activation tiles: features, ones, zeros
 struct TrainSmem {
   static constexpr int B1 = 0;                       // [64][16]

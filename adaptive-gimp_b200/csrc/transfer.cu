@@ -59,12 +59,12 @@ __device__ __forceinline__ void chunk_origin(const LevelDev& V, long long blk, i
 // warp's next item is another block.  There are no atomics on shared memory
 // (an f32 add there is a compare-and-swap loop) and no CTA barriers.
 //
-// What bounds it: instruction issue (38 warp instructions per 3D particle, half
-// of them multiply-adds, at 52 percent of the issue slots) and, between, the
+// What bounds it: instruction issue (41 warp instructions per 3D particle, half
+// of them multiply-adds, at 53 percent of the issue slots) and, between, the
 // latency of step 1's reads at 16 warps per SM.  Before (one lane per row of
 // three nodes, a 52-float record read by nine lanes, shared-memory atomics at
-// every change of cell) it took 53.  1.9M 3D particles on three levels 172 ->
-// 129 us, 15.5M 1210 -> 900, 0.6M at 8 per cell 70 -> 53, 50,000 16.6 -> 11.3;
+// every change of cell) it took 53.  1.9M 3D particles on three levels 172 (182
+// before the particles' rows) -> 129 us, 15.5M 1210 -> 900, 0.6M at 8 per cell 70 -> 53, 50,000 16.6 -> 11.3;
 // 4.1M 2D particles at 4 per cell 254 (at the best of its CTA sizes, 613 at the
 // default) -> 213 us.  Also measured: long tasks in dense cells (up to 32
 // particles: 273 us, a warp's range of items then differs in cost), the next

@@ -265,8 +265,8 @@ agimp_status agimp_set_surrogate(agimp_sim* s, const agimp_mlp* m, const float* 
 /* Training-pair recorder (snow plasticity): every substep, particles whose new
  * slot is a multiple of `stride` append (features [7], exact projected state
  * [4]) to the device arrays X [capacity][7], T [capacity][4]; X == NULL
- * switches it off.  agimp_recorded returns the number appended (it may exceed
- * capacity; only the first capacity are stored). */
+ * switches it off.  Recording changes no result.  agimp_recorded returns the
+ * number appended (it may exceed capacity; only the first capacity are stored). */
 agimp_status agimp_set_recorder(agimp_sim* s, float* X, float* T, int64_t capacity, int32_t stride);
 agimp_status agimp_recorded(agimp_sim* s, int64_t* count, int32_t reset);
 /* bit 0: a tensor-core completion wait timed out.  Synchronizes the device. */
